@@ -127,7 +127,9 @@ DevParams to_dev(const grb_params& p) {
     for (int i = 0; i < GRB_MAX_PIECES; ++i) {
       e.K[i] = p.eos.pw_kappa[i]; e.G[i] = p.eos.pw_gamma[i];
       e.R[i] = p.eos.pw_rho[i]; e.E[i] = p.eos.pw_eps[i];
+      e.iGm1[i] = 1.0 / (e.G[i] - 1.);
     }
+    e.igthm1 = 1.0 / e.gthm1;
   }
   e.ih0 = 1.0 / e.h_min;
   d.rho_fl = p.rho_fl; d.ye_fl = p.ye_fl; d.temp_fl = p.temp_fl; d.atmo_tol = p.atmo_tol;

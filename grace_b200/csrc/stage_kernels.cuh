@@ -36,43 +36,23 @@ struct StageBufs {
 };
 
 // ---- the Riemann problem at one face (grmhd.hh:774-970) -------------------
-template <int dir, bool FAST = false>
+template <int dir>
 __device__ __forceinline__ void mhd_fluxes(const DevParams& P, bool rusanov,
                                            double* pl, double* pr, const Met& m, double f[7],
                                            double vb[4]) {
   const double alp = m.alp, sqrtg = m.sqrtg;
-  double wl, wr, iwl = 0.0, iwr = 0.0;
-  if (FAST) {
-    // 1/W = rsqrt(1 + z^2), W = (1 + z^2) / W: no square root, no division
-    const double ql = 1. + sqs(m.g, pl + GRB_P_ZX), qr = 1. + sqs(m.g, pr + GRB_P_ZX);
-    iwl = rsqrt(ql);
-    iwr = rsqrt(qr);
-    wl = ql * iwl;
-    wr = qr * iwr;
-  } else {
-    wl = lorentz(m.g, pl + GRB_P_ZX);
-    wr = lorentz(m.g, pr + GRB_P_ZX);
-  }
+  const double wl = lorentz(m.g, pl + GRB_P_ZX), wr = lorentz(m.g, pr + GRB_P_ZX);
   double bl[4], br[4], b2l, b2r, vtl[3], vtr[3];
   const double gdd = dir == 0 ? m.gi[0] : dir == 1 ? m.gi[3] : m.gi[5];
   double cml, cpl, cmr, cpr, cmin, cmax;
-  const double ialp = m.ialp;  // FAST: set by make_met<true>
-  if (FAST) {
-    comoving_b_f(alp, ialp, m.beta, m.g, pl + GRB_P_BX, pl + GRB_P_ZX, wl, iwl, bl, b2l);
-    comoving_b_f(alp, ialp, m.beta, m.g, pr + GRB_P_BX, pr + GRB_P_ZX, wr, iwr, br, b2r);
-    vtilde_f(alp, m.beta, pl + GRB_P_ZX, iwl, vtl);
-    vtilde_f(alp, m.beta, pr + GRB_P_ZX, iwr, vtr);
-    char_speeds_f2(ialp, m.beta[dir], gdd, pl, pr, wl, wr, b2l, b2r, vtl[dir], vtr[dir], cml, cpl, cmr, cpr);
-  } else {
-    comoving_b(alp, m.beta, m.g, pl + GRB_P_BX, pl + GRB_P_ZX, wl, bl, b2l);
-    comoving_b(alp, m.beta, m.g, pr + GRB_P_BX, pr + GRB_P_ZX, wr, br, b2r);
-    vtilde(alp, m.beta, pl + GRB_P_ZX, wl, vtl);
-    vtilde(alp, m.beta, pr + GRB_P_ZX, wr, vtr);
-    char_speeds(alp, m.beta[dir], pl[GRB_P_RHO], pl[GRB_P_PRESS], pl[GRB_P_EPS], pl[GRB_P_CS2], wl,
-                b2l, vtl[dir], gdd, cml, cpl);
-    char_speeds(alp, m.beta[dir], pr[GRB_P_RHO], pr[GRB_P_PRESS], pr[GRB_P_EPS], pr[GRB_P_CS2], wr,
-                b2r, vtr[dir], gdd, cmr, cpr);
-  }
+  comoving_b(alp, m.beta, m.g, pl + GRB_P_BX, pl + GRB_P_ZX, wl, bl, b2l);
+  comoving_b(alp, m.beta, m.g, pr + GRB_P_BX, pr + GRB_P_ZX, wr, br, b2r);
+  vtilde(alp, m.beta, pl + GRB_P_ZX, wl, vtl);
+  vtilde(alp, m.beta, pr + GRB_P_ZX, wr, vtr);
+  char_speeds(alp, m.beta[dir], pl[GRB_P_RHO], pl[GRB_P_PRESS], pl[GRB_P_EPS], pl[GRB_P_CS2], wl,
+              b2l, vtl[dir], gdd, cml, cpl);
+  char_speeds(alp, m.beta[dir], pr[GRB_P_RHO], pr[GRB_P_PRESS], pr[GRB_P_EPS], pr[GRB_P_CS2], wr,
+              b2r, vtr[dir], gdd, cmr, cpr);
   if (rusanov) {
     cmax = fmax(fmax(fabs(cml), fabs(cmr)), fmax(fabs(cpl), fabs(cpr)));
     if (fmin(pl[GRB_P_RHO], pr[GRB_P_RHO]) < P.rusanov_c_limit)
@@ -83,11 +63,6 @@ __device__ __forceinline__ void mhd_fluxes(const DevParams& P, bool rusanov,
     cmax = fmax(0., fmax(cpl, cpr));
   }
   if (cmin < 1e-12 && cmax < 1e-12) { cmin = 1; cmax = 1; }
-  // FAST: one reciprocal for all HLL fluxes of the face
-  const double isum = FAST ? 1.0 / (cmax + cmin) : 0.0;
-  auto hll = [&](double fL, double fR, double uL, double uR, double cn, double cx) {
-    return FAST ? hll_r(fL, fR, uL, uR, cn, cx, isum) : grb::hll(fL, fR, uL, uR, cn, cx);
-  };
   if (P.emf == GRB_EMF_UCT) {
     const int a0 = dir == 0 ? 1 : 0, a1 = dir == 2 ? 1 : 2;
     vb[0] = hll(vtl[a0], vtr[a0], 0, 0, cmin, cmax);
@@ -96,9 +71,9 @@ __device__ __forceinline__ void mhd_fluxes(const DevParams& P, bool rusanov,
     vb[3] = cmax;
   }
   const ConsFlux L = cons_flux(alp, m.beta, m.g, pl[GRB_P_RHO], pl[GRB_P_PRESS], pl[GRB_P_EPS],
-                               pl + GRB_P_ZX, pl[GRB_P_ENT], wl, b2l, bl, vtl, dir, ialp);
+                               pl + GRB_P_ZX, pl[GRB_P_ENT], wl, b2l, bl, vtl, dir);
   const ConsFlux R = cons_flux(alp, m.beta, m.g, pr[GRB_P_RHO], pr[GRB_P_PRESS], pr[GRB_P_EPS],
-                               pr + GRB_P_ZX, pr[GRB_P_ENT], wr, b2r, br, vtr, dir, ialp);
+                               pr + GRB_P_ZX, pr[GRB_P_ENT], wr, b2r, br, vtr, dir);
   f[GRB_DENS] = sqrtg * hll(L.fD, R.fD, L.D, R.D, cmin, cmax);
   f[GRB_ENTROPYSTAR] = sqrtg * hll(L.fent, R.fent, L.ents, R.ents, cmin, cmax);
   f[GRB_TAU] = sqrtg * hll(L.ftau, R.ftau, L.tau, R.tau, cmin, cmax);
@@ -119,6 +94,100 @@ __device__ __forceinline__ void mhd_fluxes(const DevParams& P, bool rusanov,
       vb[0] = sqrtg * hll(Bl[1] * vtl[2] - Bl[2] * vtl[1], Br[1] * vtr[2] - Br[2] * vtr[1], Bl[1], Br[1], cmin, cmax);
       vb[1] = -sqrtg * hll(Bl[0] * vtl[2] - Bl[2] * vtl[0], Br[0] * vtr[2] - Br[2] * vtr[0], Bl[0], Br[0], cmin, cmax);
     }
+  }
+}
+
+// One side of a face (tuned mode): conserved variables U and their fluxes F
+// along dir (DENS, S_j, TAU, ENTROPYSTAR, YESTAR; undensitized), the
+// transport velocity vt, the speeds.  cons_flux, comoving_b, vtilde and
+// char_speeds in terms of the lowered z_i and B_i, with Bz = B^i z_i =
+// alpha b^0 and a = alpha/W: b_i = (B_i + Bz z_i)/W (lowered in spacetime),
+// alpha b^d = a B^d + Bz vt^d, and with S_j and tau
+//   F(S_j) = vt^d S_j - a B^d b_j + alpha p* delta_jd
+//   F(tau) = vt^d (tau + p*) + p* beta^d - a B^d Bz,
+// so no raised b^i, no lowered shift or velocity is formed.  No division or
+// square root beyond rcp_f, rsqrt_f and sqrt_f.
+struct FaceSide {
+  double U[7], F[7], vt[3], cm, cp;
+};
+template <int dir>
+__device__ __forceinline__ void face_side(const Met& m, double ia2, double gdd, const double* p, FaceSide& o) {
+  const double* z = p + GRB_P_ZX;
+  const double* B = p + GRB_P_BX;
+  double zl[3], Bl[3];
+  mvs(m.g, z, zl);
+  mvs(m.g, B, Bl);
+  const double q = 1. + (z[0] * zl[0] + z[1] * zl[1] + z[2] * zl[2]);
+  const double iW = rsqrt_f(q), W = q * iW;
+  const double Bz = B[0] * zl[0] + B[1] * zl[1] + B[2] * zl[2];
+  const double b2 = (B[0] * Bl[0] + B[1] * Bl[1] + B[2] * Bl[2] + Bz * Bz) * (iW * iW);
+  const double a = m.alp * iW;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) o.vt[i] = a * z[i] - m.beta[i];
+  const double h = p[GRB_P_RHO] * (1. + p[GRB_P_EPS]) + p[GRB_P_PRESS] + b2;
+  const double pstar = p[GRB_P_PRESS] + 0.5 * b2;
+  const double vd = o.vt[dir], aB = a * B[dir];
+  char_speeds_f(m.ialp, ia2, m.beta[dir], gdd, h, p[GRB_P_CS2], W, b2, vd, o.cm, o.cp);
+  const double D = p[GRB_P_RHO] * W, hW = h * W;
+  o.U[GRB_DENS] = D;
+  o.F[GRB_DENS] = D * vd;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const double bj = (Bl[j] + Bz * zl[j]) * iW;
+    const double S = hW * zl[j] - Bz * bj;
+    o.U[GRB_SX + j] = S;
+    o.F[GRB_SX + j] = vd * S - aB * bj + (j == dir ? m.alp * pstar : 0.0);
+  }
+  const double tau = hW * W - pstar - Bz * Bz - D;
+  o.U[GRB_TAU] = tau;
+  o.F[GRB_TAU] = vd * (tau + pstar) + pstar * m.beta[dir] - aB * Bz;
+  o.U[GRB_YESTAR] = p[GRB_P_YE] * D;
+  o.F[GRB_YESTAR] = p[GRB_P_YE] * o.F[GRB_DENS];
+  o.U[GRB_ENTROPYSTAR] = p[GRB_P_ENT] * D;
+  o.F[GRB_ENTROPYSTAR] = p[GRB_P_ENT] * o.F[GRB_DENS];
+}
+
+// mhd_fluxes in tuned mode (same functions up to rounding): the sides by
+// face_side, and the HLL combination (cmax fL + cmin fR - cmax cmin (uR -
+// uL)) sqrt(gamma) / (cmax + cmin) with its three factors formed once.
+template <int dir>
+__device__ __forceinline__ void mhd_fluxes_f(const DevParams& P, bool rusanov, const double* pl, const double* pr,
+                                             const Met& m, double f[7], double vb[4]) {
+  const double gdd = dir == 0 ? m.gi[0] : dir == 1 ? m.gi[3] : m.gi[5];
+  const double ia2 = m.ialp * m.ialp;
+  FaceSide L, R;
+  face_side<dir>(m, ia2, gdd, pl, L);
+  face_side<dir>(m, ia2, gdd, pr, R);
+  double cmin, cmax;
+  if (rusanov) {
+    cmax = fmax(fmax(fabs(L.cm), fabs(R.cm)), fmax(fabs(L.cp), fabs(R.cp)));
+    if (fmin(pl[GRB_P_RHO], pr[GRB_P_RHO]) < P.rusanov_c_limit)
+      cmax = fmax(cmax, m.alp * sqrt(gdd) + fabs(m.beta[dir]));
+    cmin = cmax;
+  } else {
+    cmin = -fmin(0., fmin(L.cm, R.cm));
+    cmax = fmax(0., fmax(L.cp, R.cp));
+  }
+  if (cmin < 1e-12 && cmax < 1e-12) { cmin = 1; cmax = 1; }
+  const double isum = rcp_f(cmax + cmin);
+  const double kl = cmax * isum * m.sqrtg, kr = cmin * isum * m.sqrtg, ku = kl * cmin;
+#pragma unroll
+  for (int v = 0; v < 7; ++v) f[v] = kl * L.F[v] + kr * R.F[v] - ku * (R.U[v] - L.U[v]);
+  const double* Bl = pl + GRB_P_BX;
+  const double* Br = pr + GRB_P_BX;
+  constexpr int t0 = dir == 0 ? 1 : 0, t1 = dir == 2 ? 1 : 2;  // the transverse axes
+  if (P.emf == GRB_EMF_UCT) {
+    vb[0] = (cmax * L.vt[t0] + cmin * R.vt[t0]) * isum;
+    vb[1] = (cmax * L.vt[t1] + cmin * R.vt[t1]) * isum;
+    vb[2] = cmin;
+    vb[3] = cmax;
+  } else {
+    // transport of the transverse B^t1 and B^t0 along dir: +-E of the third axis
+    const double s0 = dir == 1 ? -1.0 : 1.0;
+    vb[0] = s0 * (kl * (Bl[t1] * L.vt[dir] - Bl[dir] * L.vt[t1]) + kr * (Br[t1] * R.vt[dir] - Br[dir] * R.vt[t1]) -
+                  ku * (Br[t1] - Bl[t1]));
+    vb[1] = -s0 * (kl * (Bl[t0] * L.vt[dir] - Bl[dir] * L.vt[t0]) + kr * (Br[t0] * R.vt[dir] - Br[dir] * R.vt[t0]) -
+                   ku * (Br[t0] - Bl[t0]));
   }
 }
 
@@ -164,10 +233,16 @@ __device__ __forceinline__ void getflux(const DevParams& P, const Geo& G, int i,
   const double bn = FAST ? __ldg(bface + bi) * m.isqrtg : __ldg(bface + bi) / m.sqrtg;
   pl[GRB_P_BX + dir] = bn;
   pr[GRB_P_BX + dir] = bn;
+  if (FAST) {
+    eos_PT_f(P.eos, pl);
+    eos_PT_f(P.eos, pr);
+    mhd_fluxes_f<dir>(P, rusanov, pl, pr, m, f, vb);
+    return;
+  }
   uint32_t q0 = 0;
   pl[GRB_P_PRESS] = eos_PT(P.eos, pl[GRB_P_EPS], pl[GRB_P_CS2], nullptr, pl[GRB_P_TEMP], pl[GRB_P_RHO], q0);
   pr[GRB_P_PRESS] = eos_PT(P.eos, pr[GRB_P_EPS], pr[GRB_P_CS2], nullptr, pr[GRB_P_TEMP], pr[GRB_P_RHO], q0);
-  mhd_fluxes<dir, FAST>(P, rusanov, pl, pr, m, f, vb);
+  mhd_fluxes<dir>(P, rusanov, pl, pr, m, f, vb);
 }
 
 __device__ __forceinline__ void store_face(const Geo& G, const StageBufs& B, int emf_kind, int dir,
