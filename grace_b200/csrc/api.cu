@@ -138,7 +138,7 @@ DevParams to_dev(const grb_params& p) {
   d.beta_fallback = p.beta_fallback; d.alp_bh_thresh = p.alp_bh_thresh;
   d.use_ent_backup = p.use_ent_backup;
   d.rusanov_c_limit = p.rusanov_use_c_limit;
-  d.fofc = p.fofc_enable; d.dmp_enable = p.dmp_enable; d.dmp_M = p.dmp_M;
+  d.fofc = p.fofc_enable; d.dmp_enable = p.dmp_enable; d.dmp_M = p.dmp_M; d.idmp_M = 1.0 / p.dmp_M;
   d.recon = p.recon; d.riemann = p.riemann; d.emf = p.emf;
   return d;
 }
@@ -483,8 +483,8 @@ void launch_aux_deferred(unsigned nb, cudaStream_t s, const DevParams& P, const 
                          const double* bx, const double* by, const double* bz, double* aux, const double* idx,
                          const double* crd, const StageBufs& B, const DtArgs& dta) {
   cudaMemsetAsync(B.nadefer, 0, sizeof(unsigned long long), s);
-  k_aux_front<MINB, kDt, true><<<nb, 128, 0, s>>>(P, G, b, st, bx, by, bz, aux, idx, crd, B, dta);
-  k_aux_backup<MINB, kDt, true><<<std::min(nb, 148u * 8u), 128, 0, s>>>(P, G, st, bx, by, bz, aux, idx, crd, B,
+  k_aux_front<MINB, kDt><<<nb, 128, 0, s>>>(P, G, b, st, bx, by, bz, aux, idx, crd, B, dta);
+  k_aux_backup<MINB, kDt><<<std::min(nb, 148u * 8u), 128, 0, s>>>(P, G, st, bx, by, bz, aux, idx, crd, B,
                                                                        dta);
 }
 
@@ -1241,13 +1241,13 @@ int launch_c2p(grb_handle* h, int64_t n, const double* cons, const double* metri
     }
     CK(cudaMemsetAsync(h->d_ndefer, 0, sizeof(unsigned long long), s));
     if (learned)
-      k_c2p_batch_front<true, true><<<nb, kC2PThreads, 0, s>>>(h->dp, n, cons, metric, prims, cons_out, err, d,
+      k_c2p_batch_front<true><<<nb, kC2PThreads, 0, s>>>(h->dp, n, cons, metric, prims, cons_out, err, d,
                                                               h->d_mlp_pack, h->d_flags, h->d_defer, h->d_ndefer);
     else
-      k_c2p_batch_front<false, true><<<nb, kC2PThreads, 0, s>>>(h->dp, n, cons, metric, prims, cons_out, err, d,
+      k_c2p_batch_front<false><<<nb, kC2PThreads, 0, s>>>(h->dp, n, cons, metric, prims, cons_out, err, d,
                                                                nullptr, h->d_flags, h->d_defer, h->d_ndefer);
     const unsigned gb = (unsigned)std::min<int64_t>(nb, 148 * 16);
-    k_c2p_batch_backup<true><<<gb, kC2PThreads, 0, s>>>(h->dp, n, metric, prims, cons_out, err, h->d_flags,
+    k_c2p_batch_backup<<<gb, kC2PThreads, 0, s>>>(h->dp, n, metric, prims, cons_out, err, h->d_flags,
                                                        h->d_defer, h->d_ndefer);
     h->launches += 2;
     CK(cudaGetLastError());

@@ -444,34 +444,6 @@ GRB_HD WB wb_of(const Met& m, const double pr[13]) {
   o.b2 = (sqs(m.g, B) + o.Bz * o.Bz) * o.iW * o.iW;
   return o;
 }
-// prims_to_cons from a cached WB; with `need` holding no ERR_RESET_STILDE
-// or ERR_RESET_TAU bit the momenta and tau (and b^mu) are not formed (D,
-// Ye* and the entropy density always are).
-GRB_HD void prims_to_cons_wb(const double pr[13], double c[10], const Met& m, const WB& q, double ialp,
-                             uint32_t need) {
-  const double D = pr[GRB_P_RHO] * q.W;
-  c[0] = m.sqrtg * D;
-  c[6] = m.sqrtg * (pr[GRB_P_ENT] * D);
-  c[5] = c[0] * pr[GRB_P_YE];
-  if (need & (ERR_RESET_STILDE | ERR_RESET_TAU)) {
-    const double b0 = q.Bz * ialp;
-    double b[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-      b[i] = (pr[GRB_P_BX + i] + m.alp * b0 * (pr[GRB_P_ZX + i] - q.W * m.beta[i] * ialp)) * q.iW;
-    const double rhoh = pr[GRB_P_RHO] * (1. + pr[GRB_P_EPS]) + pr[GRB_P_PRESS] + q.b2;
-    const double pstar = pr[GRB_P_PRESS] + 0.5 * q.b2;
-    double bl[3], betal[3], zl[3];
-    mvs(m.g, b, bl);
-    mvs(m.g, m.beta, betal);
-    mvs(m.g, pr + GRB_P_ZX, zl);
-    const double tau = rhoh * q.W * q.W - pstar - m.alp * m.alp * b0 * b0 - D;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) c[1 + i] = m.sqrtg * (rhoh * q.W * zl[i] - m.alp * b0 * (bl[i] + betal[i] * b0));
-    c[4] = m.sqrtg * tau;
-  }
-}
-
 GRB_HD void handle_sig(uint32_t sig, bool lenient, uint32_t& err, uint32_t& fatal) {
   if (sig & SIG_RHO_HIGH) {
     err |= ERR_SIG_RHO_HIGH | ERR_ALL_RESETS;
@@ -525,25 +497,28 @@ struct C2POut {
   double W, iW;  // Lorentz factor of the final primitives (tuned mode)
 };
 
-// conservs_to_prims (c2p.cpp:188-414), in three parts so that a batch can
-// defer the entropy backup of the states that need it to a second pass
-// (c2p_front: up to the decision to distrust the Kastaun result;
-// c2p_backup: the entropy-based solve; c2p_back: signals, atmosphere,
-// temperature floor, limit_primitives, prims_to_cons).  c2p() runs the three
-// in sequence: the reference's order of operations.  c: densitized cons
-// with densitized cell-centred B (in), re-densitized consistent cons (out).
-// FAST (tuned mode): multiplications by 1/sqrt(gamma) and 1/D where the
-// reference divides repeatedly by the same value, the FAST master function,
-// and W, b^mu, b^2 formed once per set of primitives (WB) instead of in
-// each of the beta test, limit_primitives and prims_to_cons; equal to the
-// reference's operations up to rounding.  kAllCons false (tuned mode):
-// the returned cons hold only what the reset flags in o.err ask for.
+// conservs_to_prims (c2p.cpp:188-414), in three parts (c2p_front: up to the
+// decision to distrust the Kastaun result; c2p_backup: the entropy-based
+// solve; c2p_back: signals, atmosphere, temperature floor, limit_primitives,
+// prims_to_cons).  c2p() runs the three in sequence: the reference's order of
+// operations.  c: densitized cons with densitized cell-centred B (in),
+// re-densitized consistent cons (out).  FAST (the tuned mode's learned
+// bracket; its plain bracket takes c2p_front_f below): multiplications by
+// 1/sqrt(gamma) and 1/D where the reference divides repeatedly by the same
+// value, the FAST master function, and W, b^mu, b^2 formed once per set of
+// primitives (WB) instead of in each of the beta test, limit_primitives and
+// prims_to_cons; equal to the reference's operations up to rounding.
 struct C2PState {
   C2POut o;
   uint32_t ret;
   bool failed, lenient, ran, backup, done;
   WB wb;
   bool wb_ok;  // wb belongs to the current z and B
+  // c2p_front_f: the top of the Kastaun bracket (0: not formed), and whether
+  // prims' entropy is set (otherwise that slot holds the thermal energy, from
+  // which c2p_back_f forms it)
+  double mu0;
+  bool ent_ok;
 };
 
 template <bool FAST = false>
@@ -552,6 +527,7 @@ GRB_HD C2PState c2p_front(double c[10], double pr[13], const Met& m, const DevPa
   C2PState F{};
   F.o = C2POut{0u, 0u, 0, false, false, 0.0, 0.0, 0.0};
   F.wb_ok = false;
+  F.ent_ok = true;
   F.failed = false;
   F.ret = 0;
   const DevEos& e = P.eos;
@@ -643,12 +619,10 @@ GRB_HD void c2p_backup(C2PState& F, double c[10], double pr[13], const Met& m, c
 
 // kDry: a dry run (the FOFC flag's), which needs only o.floored: the final
 // prims_to_cons is skipped.
-template <bool FAST = false, bool kAllCons = true, bool kDry = false>
+template <bool kDry = false>
 GRB_HD void c2p_back(C2PState& F, double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph) {
   const DevEos& e = P.eos;
   C2POut& o = F.o;
-  WB& wb = F.wb;
-  const double ialp = FAST ? 1.0 / m.alp : 0.0;
   if (F.ran) {
     const uint32_t ret = F.ret;
     if (ret & (SIG_EPS_HIGH | SIG_RHO_LOW | SIG_RHO_HIGH | SIG_VEL_HIGH)) o.floored = true;
@@ -659,7 +633,6 @@ GRB_HD void c2p_back(C2PState& F, double c[10], double pr[13], const Met& m, con
   if (F.failed || excise || pr[GRB_P_RHO] < (1. + P.atmo_tol) * P.rho_fl) {
     reset_atmo(c, pr, m, P, o.err);
     o.floored = true;
-    F.wb_ok = false;
   } else if (pr[GRB_P_TEMP] < P.temp_fl) {
     pr[GRB_P_TEMP] = P.temp_fl;
     double cs2;
@@ -671,22 +644,15 @@ GRB_HD void c2p_back(C2PState& F, double c[10], double pr[13], const Met& m, con
   } else {  // limit_primitives (c2p.cpp:63-115)
     uint32_t s2 = 0;
     const double z2max = P.max_w * P.max_w - 1.;
-    if (FAST && !F.wb_ok) { wb = wb_of(m, pr); F.wb_ok = true; }
-    const double z2 = FAST ? wb.z2 : sqs(m.g, pr + GRB_P_ZX);
+    const double z2 = sqs(m.g, pr + GRB_P_ZX);
     if (z2 >= z2max) {
       const double zn = 0.99 * sqrt(z2max / z2);
       pr[GRB_P_ZX] *= zn; pr[GRB_P_ZY] *= zn; pr[GRB_P_ZZ] *= zn;
       s2 |= SIG_VEL_HIGH;
-      if (FAST) wb = wb_of(m, pr);
     }
-    double b2;
-    if (FAST) {
-      b2 = wb.b2;
-    } else {
-      const double W = lorentz(m.g, pr + GRB_P_ZX);
-      double b[4];
-      comoving_b(m.alp, m.beta, m.g, pr + GRB_P_BX, pr + GRB_P_ZX, W, b, b2);
-    }
+    const double W = lorentz(m.g, pr + GRB_P_ZX);
+    double b[4], b2;
+    comoving_b(m.alp, m.beta, m.g, pr + GRB_P_BX, pr + GRB_P_ZX, W, b, b2);
     const double sigma = b2 / pr[GRB_P_RHO];
     if (sigma >= P.max_sigma) {
       pr[GRB_P_RHO] *= 1.001 * sigma / P.max_sigma;
@@ -698,33 +664,589 @@ GRB_HD void c2p_back(C2PState& F, double c[10], double pr[13], const Met& m, con
     handle_sig(s2, F.lenient, o.err, o.fatal);
     if (s2 & (SIG_VEL_HIGH | SIG_SIGMA_HIGH)) o.floored = true;
   }
-  if (kDry) return;
-  if (FAST) {
-    if (!F.wb_ok) wb = wb_of(m, pr);
-    prims_to_cons_wb(pr, c, m, wb, ialp, kAllCons ? ~0u : o.err);
-    o.W = wb.W;
-    o.iW = wb.iW;
-  } else {
-    prims_to_cons(pr, c, m);
-  }
+  if (!kDry) prims_to_cons(pr, c, m);
 }
 
-template <bool FAST = false, bool kAllCons = true>
 GRB_HD C2POut c2p(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph,
                   bool dry_run, double alp_bh_thresh, const Guess& gs) {
-  C2PState F = c2p_front<FAST>(c, pr, m, P, dry_run, alp_bh_thresh, gs);
+  C2PState F = c2p_front(c, pr, m, P, dry_run, alp_bh_thresh, gs);
   if (F.done) return F.o;
   if (F.backup) c2p_backup(F, c, pr, m, P);
-  c2p_back<FAST, kAllCons>(F, c, pr, m, P, r_sph);
+  c2p_back(F, c, pr, m, P, r_sph);
   return F.o;
 }
 // The FOFC flag's dry run (c2p.cpp:188-414 with the dry-run flag): whether
 // the state would be floored; no entropy backup, no final prims_to_cons.
-template <bool FAST = false>
 GRB_HD bool c2p_floored(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph) {
-  C2PState F = c2p_front<FAST>(c, pr, m, P, true, 1e30, no_guess());
+  C2PState F = c2p_front(c, pr, m, P, true, 1e30, no_guess());
   if (F.done) return F.o.floored;
-  c2p_back<FAST, true, true>(F, c, pr, m, P, r_sph);
+  c2p_back<true>(F, c, pr, m, P, r_sph);
+  return F.o.floored;
+}
+
+// ---- the c2p of the tuned mode ----------------------------------------------
+// The same functions and decisions as c2p_front, c2p_backup and c2p_back
+// above, equal up to rounding, arranged for the GPU.  What bound the direct
+// form was not FP64 throughput (27 % of the pipe) but instruction count and
+// fetch: the master function inlined at each of its call sites, every
+// division and root with its slow-path branch, min/max sequences, the
+// transcendental calls of three equation-of-state branches.  Here
+//  - each root solve evaluates its function at one place;
+//  - the function's quotients and roots are rcp_f, rsqrt_f: W = rsqrt(1 - v^2),
+//    W/(1+W) = 1/(1 + 1/W), P/rho without rho for the ideal gas;
+//  - the Kastaun scalars are formed once, limit_conservatives' among them, and
+//    B.z = W mu (r.B), so W, B.z and b^2 of the solution need no contraction;
+//  - the primitives' replacements (atmosphere, temperature floor,
+//    magnetisation limit) share one equation-of-state evaluation, and the
+//    entropy is formed once, at the end.
+
+// Scalars of one state (kastaun_c2p.hh:306-337): D, 1/D, D^(-1/2), q = tau/D,
+// r^2, b^2 = B^2/D, (r.b)^2 and r^2 b^2 minus it, r.b.
+struct KScF {
+  double D, iD, isD, q, r2, b2, rb2, bro, rBt;
+  double ow, vmax;  // 1 - v_max^2 = 1 / (1 + r^2 / h0^2), v_max^2
+};
+// kRound: quotients and root correctly rounded, in the reference's order, for
+// the plain mode's iterates (W^2 / f', 10^5 in fast magnetised flows,
+// amplifies their rounding in the primitives).
+template <bool kRound>
+GRB_HD void kscf(const DevEos& e, const Met& m, const double c[10], KScF& k) {
+  k.D = c[0];
+  k.iD = kRound ? 1.0 / k.D : rcp_f(k.D);
+  k.q = c[4] * k.iD;
+  const double isD = kRound ? 1.0 / sqrt(k.D) : rsqrt_f(k.D);
+  double r[3], Bt[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) { r[i] = c[1 + i] * k.iD; Bt[i] = c[7 + i] * isD; }
+  k.r2 = sqs(m.gi, r);
+  k.b2 = sqs(m.g, Bt);
+  k.rBt = r[0] * Bt[0] + r[1] * Bt[1] + r[2] * Bt[2];
+  k.rb2 = k.rBt * k.rBt;
+  k.bro = k.r2 * k.b2 - k.rb2;
+  k.isD = isD;
+  // v^2 is compared with v_max^2 itself: cold flows lie within rounding of it,
+  // which 1 - v^2 would lose
+  const double zs = k.r2 * (e.ih0 * e.ih0);
+  k.vmax = zs / (1.0 + zs);
+  k.ow = rcp_f(1.0 + zs);
+}
+
+// Cold part of the hybrid EOS at rho: P_cold / rho and eps_cold.
+GRB_HD void pw_cold_f(const DevEos& e, double& rho, double irho, double& pr, double& ec) {
+  const int i = pw_idx(e, rho);
+  pr = e.G[i] == 2.0 ? e.K[i] * rho : e.K[i] * pw_pow(rho, e.G[i]) * irho;
+  ec = e.E[i] + pr * e.iGm1[i];
+}
+GRB_HD double clamp_f(double x, double lo, double hi) {
+  // as fmin(hi, fmax(lo, x)): the bound for a NaN
+  x = x > lo ? x : lo;
+  return x < hi ? x : hi;
+}
+
+// Kastaun's master function at mu (kastaun_c2p.hh:122-295); the members
+// keep what the solution needs.  raw: eps before its clamps; eth: eps -
+// eps_cold (hybrid) or eps (ideal gas); prho: P / rho.
+struct KFn {
+  const DevEos* e;
+  const KScF* k;
+  double x, w, iw, rho, eps, raw, lo, eth, prho;
+  bool vhigh;
+  GRB_HD double operator()(double mu) {
+    x = rcp_f(1. + mu * k->b2);
+    const double rf = x * (k->r2 * x + mu * (x + 1.0) * k->rb2);
+    const double mx = mu * x;
+    const double qf = k->q - 0.5 * (k->b2 + mx * mx * k->bro);
+    const double rmu = rf * mu;
+    const double vsqr = rmu * mu;
+    vhigh = vsqr > k->vmax;
+    const double om = vhigh ? k->ow : 1. - vsqr;
+    w = rsqrt_f(om);
+    iw = om * w;
+    raw = w * (qf - rmu * (1.0 - mu * rcp_f(1.0 + iw)));
+    rho = k->D * iw;
+    if (e->kind == GRB_EOS_IDEAL_GAS) {
+      lo = 0.0;
+      eps = clamp_f(raw, 0.0, e->eps_max);
+      eth = eps;
+      prho = e->gm1 * eps;
+    } else {
+      double irho = w * k->iD, pr, ec;
+      if (rho > e->rhomax || rho < e->rhomin) irho = rcp_f(clamp_f(rho, e->rhomin, e->rhomax));
+      double r = clamp_f(rho, e->rhomin, e->rhomax);
+      pw_cold_f(*e, r, irho, pr, ec);
+      lo = ec < e->eps_max ? ec : e->eps_max;
+      eps = clamp_f(raw, lo, e->eps_max);
+      eth = eps - ec;
+      prho = pr + eth * e->gthm1;
+    }
+    const double h = 1. + eps + prho, e1 = 1. + eps;
+    const double qa = 1. + qf - rmu;
+    // nu = max(h qa / (1 + eps), h / W)
+    const bool a = qa >= iw * e1;
+    const double num = a ? e1 : 1.0;
+    return mu - num * rcp_f(h * (a ? qa : iw) + rmu * num);
+  }
+  GRB_HD void clamp() {}
+};
+
+// The entropy-based master function at mu (ent_based_c2p.hh:44-170) with
+// the thermal energy eth = exp(Gamma' (s + log rho)), Gamma' = Gamma - 1 or
+// Gamma_th - 1: with s + log D in sl and log(rho/D) = log(1 - v^2)/2, one
+// logarithm and one exponential an evaluation.
+struct EFn {
+  const DevEos* e;
+  const KScF* k;
+  double sl, g, elo;  // elo: the least thermal energy
+  double x, w, iw, rho, eps, eth, raw, hi, prho;
+  bool vhigh;
+  GRB_HD double operator()(double mu) {
+    x = rcp_f(1. + mu * k->b2);
+    const double rf = x * (k->r2 * x + mu * (x + 1.0) * k->rb2);
+    const double rmu = rf * mu;
+    const double vsqr = rmu * mu;
+    vhigh = vsqr > k->vmax;
+    const double om = vhigh ? k->ow : 1. - vsqr;
+    w = rsqrt_f(om);
+    iw = om * w;
+    rho = k->D * iw;
+    double lr = 0.5 * log(om), pr = 0.0, ec = 0.0;
+    if (e->kind != GRB_EOS_IDEAL_GAS) {
+      double irho = w * k->iD;
+      double r = rho;
+      if (rho > e->rhomax || rho < e->rhomin) {
+        r = clamp_f(rho, e->rhomin, e->rhomax);
+        irho = rcp_f(r);
+        lr = log(r * k->iD);
+      }
+      pw_cold_f(*e, r, irho, pr, ec);
+    }
+    raw = exp(g * (sl + lr));
+    hi = e->eps_max - ec;
+    eth = raw > elo ? raw : elo;
+    eth = eth < hi ? eth : hi;
+    eps = ec + eth;
+    prho = pr + eth * g;
+    return mu - rcp_f((1. + eps + prho) * iw + rmu);
+  }
+  // keeps s in its range at the density last visited
+  GRB_HD void clamp() {
+    if (eth != raw) sl = log(eth) / g + log(k->D) - log(clamp_f(rho, e->rhomin, e->rhomax));
+  }
+};
+
+// Root of an increasing f with f(0) < 0 by the secant method from x (first
+// step along slope 1, which f approaches for slow flows), kept inside the
+// bracket that the signs give (else its midpoint); past kSecantMax steps it
+// bisects.  Ends when the next step is below eps of x, or f below its own
+// rounding: 1 - v^2 carries an error of eps/2, which W^2 amplifies, and where
+// f' is small (1/100 in fast magnetised flows) a step repeats at that level
+// without shrinking; the slope is not taken from differences near it.  So the
+// primitives are as close to the sampled hybrid states' as Brent's (median
+// error 2.5e-13 in rho against 2.7e-13, backup solve 8.0e-14 against
+// 9.2e-14), in 3.1 evaluations on the blast wave's states where Brent from
+// [0, mu0] takes 6, 5.3 on the sampled states instead of 8.  f's members belong to the returned x.  NaN ends it.  clamp:
+// f is first visited at 0 and at x and f.clamp() called.
+constexpr int kSecantMax = 40;
+template <class Fn>
+GRB_HD double secant_root(Fn& f, double x, double top, bool clamp, int& iters, double& res) {
+  const double eps = 2.220446049250313e-16, x0 = x;
+  double lo = 0.0, hi = top, xp = 0.0, fp = 0.0, is = 1.0, ap = 1e300;
+  if (clamp) x = 0.0;
+  for (int it = clamp ? -2 : 0;; ++it) {
+    const double fx = f(x);
+    res = fx;
+    if (it < 0) {
+      f.clamp();
+      x = x0;
+      continue;
+    }
+    if (!(fx == fx)) break;
+    const double noise = (0.06 * eps) * x * (f.w * f.w);
+    const double df = fx - fp, af = fabs(fx);
+    if (it > 0 && fabs(df) > 280.0 * noise) is = (x - xp) * rcp_f(df);
+    const double d = fx * is, a = fabs(d);
+    if (it < kSecantMax ? (a <= eps * x || af <= noise || (af < 140.0 * noise && a >= 0.5 * ap))
+                        : (hi - lo <= eps * x || it > 3 * kSecantMax))
+      break;
+    if (fx > 0.0) hi = x; else lo = x;
+    ap = a;
+    xp = x;
+    fp = fx;
+    x -= d;
+    if (!(x > lo && x < hi) || it >= kSecantMax) x = 0.5 * (lo + hi);
+    ++iters;
+  }
+  return x;
+}
+
+// brent() from [0, top] with f evaluated at one place, and once more at the
+// root so that f's members belong to it.  For callers that want the plain
+// mode's iterates: the root then is the plain solve's own, to the last place
+// in most states, where two converged solvers differ by Brent's 1e-15.
+template <class Fn>
+GRB_HD double brent_root(Fn& f, double top, bool clamp, int& iters, double& res) {
+  const double macheps = 2.220446049250313e-16;
+  double sa = 0.0, sb = 0.0, fa = 0.0, fb = 0.0, c = 0.0, fc = 0.0, e = 0.0, d = 0.0;
+  bool last = false;
+  for (int it = -2;; ++it) {
+    const double fx = f(sb);
+    if (last) {
+      res = fx;
+      break;
+    }
+    if (it < 0 && clamp) f.clamp();
+    if (it == -2) {
+      fa = fx;
+      sb = top;
+      continue;
+    }
+    fb = fx;
+    if (it == -1) {
+      c = sa; fc = fa; e = sb - sa; d = e;
+    } else {
+      ++iters;
+      if ((0.0 < fb && 0.0 < fc) || (fb <= 0.0 && fc <= 0.0)) {
+        c = sa; fc = fa; e = sb - sa; d = e;
+      }
+    }
+    if (fabs(fc) < fabs(fb)) {
+      sa = sb; sb = c; c = sa;
+      fa = fb; fb = fc; fc = fa;
+    }
+    const double tol = 2.0 * macheps * fabs(sb) + 1e-15;
+    const double m = 0.5 * (c - sb);
+    if (fabs(m) <= tol || fb == 0.0 || it >= kBrentMaxIter) {
+      last = true;
+      continue;
+    }
+    if (fabs(e) < tol || fabs(fa) <= fabs(fb)) {
+      e = m; d = e;
+    } else {
+      const double ifa = rcp_f(fa);
+      double s = fb * ifa, p, q;
+      if (sa == c) {
+        p = 2.0 * m * s;
+        q = 1.0 - s;
+      } else {
+        const double ifc = rcp_f(fc);
+        q = fa * ifc;
+        const double r = fb * ifc;
+        p = s * (2.0 * m * q * (q - r) - (sb - sa) * (r - 1.0));
+        q = (q - 1.0) * (r - 1.0) * (s - 1.0);
+      }
+      if (0.0 < p) q = -q; else p = -p;
+      s = e; e = d;
+      if (2.0 * p < 3.0 * m * q - fabs(tol * q) && p < fabs(0.5 * s * q)) d = p * rcp_f(q);
+      else { e = m; d = e; }
+    }
+    sa = sb; fa = fb;
+    if (tol < fabs(d)) sb = sb + d;
+    else if (0.0 < m) sb = sb + tol;
+    else sb = sb - tol;
+  }
+  return sb;
+}
+
+// kastaun_mu0 (kastaun_c2p.hh:355-369): 1/h0, or for r >= h0 the root of
+// mu sqrt(h0^2 + rbar^2(mu)) = 1 by newton_br's iteration from the same
+// bracket, the auxiliary function evaluated at one place.
+GRB_HD double mu0_f(const DevEos& e, const KScF& k) {
+  const double h02 = e.h_min * e.h_min;
+  if (!(k.r2 >= h02)) return e.ih0;
+  double a = 0.0, b = 0.0, fa = 0.0, fb = 0.0, x = e.ih0, xold = 0.0, mu0 = e.ih0;
+  for (int it = -3; it < 30; ++it) {
+    const double xx = rcp_f(1. + x * k.b2), x2 = xx * xx;
+    const double u = h02 + xx * (k.r2 * xx + x * (xx + 1.0) * k.rb2);
+    const double ihw = rsqrt_f(u);
+    if (it == -3) {  // the bracket
+      a = rcp_f(h02 + k.r2) * (1 - 1e-10);
+      b = ihw * (1 + 1e-10);
+      if (b <= a) { a = 0.0; b = e.ih0 * (1.0 + 1e-10); }
+      x = a;
+      continue;
+    }
+    const double f = x * (u * ihw) - 1.;
+    if (it == -2) {
+      fa = f;
+      x = b;
+      continue;
+    }
+    if (it == -1) {
+      fb = f;
+      if (fa * fb > 0) break;
+      x = (fb * a - fa * b) * rcp_f(fb - fa);
+      continue;
+    }
+    const double df = (h02 + xx * (x2 * k.r2 + x * (1 + xx + x2) * k.rb2)) * ihw;
+    xold = x;
+    if (f * fb > 0) { fb = f; b = x; }
+    else if (f * fa > 0) { fa = f; a = x; }
+    x -= f * rcp_f(df);
+    if (fabs(x - xold) < 2. * 2.220446049250313e-16 * fabs(x) + 1e-10 || f == 0) {
+      mu0 = x * (1 + 1e-10);
+      break;
+    }
+    if (x > b || x < a) x = 0.5 * (b + a);
+  }
+  return mu0;
+}
+
+// Writes the primitives of a solution (Kastaun's or the entropy's) and its
+// W, B.z and b^2.
+template <class Fn>
+GRB_HD void take_solution(const DevEos& e, const Met& m, const KScF& k, const Fn& f, double mu, const double c[10],
+                          double pr[13], WB& wb, bool& wb_ok) {
+  const double rho = clamp_f(f.rho, e.rhomin, e.rhomax);
+  pr[GRB_P_RHO] = rho;
+  pr[GRB_P_EPS] = f.eps;
+  pr[GRB_P_PRESS] = f.prho * rho;
+  pr[GRB_P_TEMP] = e.kind == GRB_EOS_IDEAL_GAS ? f.eth * e.gm1 : fmax(0.0, f.eth * e.gthm1);
+  double rup[3];
+  mvs(m.gi, c + 1, rup);
+  const double kz = f.w * mu * f.x, kb = mu * k.rBt * k.isD;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) pr[GRB_P_ZX + i] = kz * (rup[i] * k.iD + kb * c[7 + i]);
+  wb.W = f.w;
+  wb.iW = f.iw;
+  wb.z2 = f.w * f.w - 1.0;
+  wb.Bz = f.w * mu * (k.rBt * (k.isD * k.D));
+  wb.b2 = (k.b2 * k.D + wb.Bz * wb.Bz) * (f.iw * f.iw);
+  wb_ok = !f.vhigh;
+}
+
+// c2p_front in the tuned mode (plain bracket).
+// kBrent: the root by Brent's iteration from the plain bracket (the batch
+// entry points), else by secant_root (the stage passes).
+template <bool kBrent, bool kDry = false>
+GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const DevParams& P, double alp_bh_thresh) {
+  C2PState F{};
+  const DevEos& e = P.eos;
+  C2POut& o = F.o;
+  o.err = ERR_RESET_ENTROPY;
+  F.failed = true;
+#pragma unroll
+  for (int v = 0; v < 10; ++v) c[v] *= m.isqrtg;
+  pr[GRB_P_BX] = c[7]; pr[GRB_P_BY] = c[8]; pr[GRB_P_BZ] = c[9];
+  F.lenient = m.alp < alp_bh_thresh;
+  if (c[0] < 0) return F;  // c2p_back_f resets it to the atmosphere
+  KScF k;
+  kscf<kBrent>(e, m, c, k);
+  double ye = c[5] * k.iD;
+  if (ye > e.yemax) { ye = e.yemax; o.err |= ERR_RESET_YE; }
+  if (ye < 0.0) { ye = 0.0; o.err |= ERR_RESET_YE; }
+  pr[GRB_P_YE] = ye;
+  // limit_conservatives (c2p.cpp:117-157); the least eps is never negative
+  const double B2 = sqs(m.g, c + 7);
+  if (k.q - 0.5 * B2 * k.iD < 0.0) {
+    double lo, hi;
+    eos_eps_range(e, lo, hi, c[0]);
+    c[4] = lo * c[0] + 0.5 * B2;
+    k.q = c[4] * k.iD;
+    o.err |= ERR_RESET_TAU;
+    o.floored = true;
+  }
+  const double qd = k.q + 1;
+  if (k.r2 > qd * qd) {
+    const double f = sqrt(qd * qd / k.r2);
+    c[1] *= f; c[2] *= f; c[3] *= f;
+    kscf<kBrent>(e, m, c, k);
+    o.err |= ERR_RESET_STILDE;
+    o.floored = true;
+  }
+  if (o.floored && kDry) {
+    F.done = true;
+    return F;
+  }
+  if (!(c[0] >= P.rho_fl * (1 + P.atmo_tol))) return F;
+  F.ran = true;
+  KFn f;
+  f.e = &e;
+  f.k = &k;
+  F.mu0 = mu0_f(e, k);
+  double res, mu;
+  if (kBrent) {
+    mu = brent_root(f, F.mu0, false, o.iters, res);
+  } else {
+    // from 1/h of the fluid at rest for slow flows, else from the bracket's
+    // top, which fast flows come close to
+    double start = F.mu0;
+    if (k.r2 < e.h_min * e.h_min) {
+      const double eps0 = k.q - 0.5 * k.b2;
+      start = fmin(start, rcp_f(1.0 + (e.kind == GRB_EOS_IDEAL_GAS ? e.g : 1.0 + e.gthm1) * fmax(eps0, 0.0)));
+    }
+    mu = secant_root(f, start, e.ih0 * (1 + 1e-10), false, o.iters, res);
+  }
+  o.mu = mu;
+  // the signals of the full evaluation (kastaun_c2p.hh:245-290)
+  if (f.vhigh) F.ret |= SIG_VEL_HIGH;
+  if (f.rho >= e.rhomax) F.ret |= SIG_RHO_HIGH;
+  else if (f.rho <= e.rhomin) F.ret |= SIG_RHO_LOW;
+  if (f.raw >= e.eps_max) F.ret |= SIG_EPS_HIGH;
+  else if (f.raw < f.lo) F.ret |= SIG_EPS_LOW;
+  F.failed = !(fabs(res) <= P.tol) || (F.ret & (SIG_RHO_HIGH | SIG_EPS_HIGH));
+  if (kDry) {
+    // only rho, T, z^2 and b^2 decide whether the state is floored
+    pr[GRB_P_RHO] = clamp_f(f.rho, e.rhomin, e.rhomax);
+    pr[GRB_P_TEMP] = e.kind == GRB_EOS_IDEAL_GAS ? f.eth * e.gm1 : f.eth * e.gthm1;
+    F.wb.z2 = f.w * f.w - 1.0;
+    F.wb.Bz = f.w * mu * (k.rBt * (k.isD * k.D));
+    F.wb.b2 = (k.b2 * k.D + F.wb.Bz * F.wb.Bz) * (f.iw * f.iw);
+    F.wb_ok = true;
+    return F;
+  }
+  take_solution(e, m, k, f, mu, c, pr, F.wb, F.wb_ok);
+  pr[GRB_P_ENT] = f.eth;
+  if (!F.wb_ok) {
+    F.wb = wb_of(m, pr);
+    F.wb_ok = true;
+  }
+  const bool distrust =
+      F.failed || (F.ret & SIG_EPS_LOW) || 2.0 * pr[GRB_P_PRESS] <= P.beta_fallback * fmax(F.wb.b2, 1e-50);
+  F.backup = distrust && P.use_ent_backup;
+  return F;
+}
+
+// c2p_backup in the tuned mode.  The reference's solve clamps the entropy to
+// its range at every density it visits and keeps it clamped: the range at
+// the bracket's two ends, its largest and smallest density, covers all.
+template <bool kBrent>
+GRB_HD void c2p_backup_f(C2PState& F, double c[10], double pr[13], const Met& m, const DevParams& P) {
+  const DevEos& e = P.eos;
+  const bool ideal = e.kind == GRB_EOS_IDEAL_GAS;
+  KScF k;
+  kscf<kBrent>(e, m, c, k);
+  const double mu0 = F.mu0 > 0.0 ? F.mu0 : mu0_f(e, k);
+  EFn f;
+  f.e = &e;
+  f.k = &k;
+  f.g = ideal ? e.gm1 : e.gthm1;
+  f.elo = ideal ? e.ent_min : e.entropy_min;
+  const double lD = log(k.D), s0 = c[6] * k.iD;
+  f.sl = s0 + lD;
+  // whether any density of the bracket may leave the entropy's range: the
+  // thermal energy at rho = D, and a lower bound of it at D/W
+  const double E0 = exp(f.g * f.sl);
+  double pr0 = 0.0, ec0 = 0.0, r0 = k.D;
+  if (!ideal) pw_cold_f(e, r0, k.iD, pr0, ec0);
+  const bool clamp = !(E0 * k.ow >= f.elo && E0 <= e.eps_max - ec0 && f.g <= 2.0);
+  int it = 0;
+  double res;
+  const double mu = kBrent ? brent_root(f, mu0, clamp, it, res)
+                           : secant_root(f, mu0, e.ih0 * (1 + 1e-10), clamp, it, res);
+  if (fabs(res) <= P.tol && f.eps < e.eps_max) {
+    uint32_t sig = 0;
+    if (f.vhigh) sig |= SIG_VEL_HIGH;
+    if (f.rho >= e.rhomax) sig |= SIG_RHO_HIGH;
+    else if (f.rho <= e.rhomin) sig |= SIG_RHO_LOW;
+    if (f.raw < f.elo * (1 - 1e-12)) sig |= SIG_ENT_LOW;
+    if (f.raw > f.hi * (1 + 1e-12)) sig |= SIG_ENT_HIGH;
+    F.ret = sig;
+    F.failed = false;
+    F.o.err |= ERR_ENT_BACKUP;
+    take_solution(e, m, k, f, mu, c, pr, F.wb, F.wb_ok);
+    pr[GRB_P_ENT] = clamp ? f.sl - lD : s0;
+    F.ent_ok = true;
+  }
+  // otherwise the Kastaun primitives stand, or the state is reset if that failed
+}
+
+// c2p_back in the tuned mode.
+template <bool kAllCons = true, bool kDry = false>
+GRB_HD void c2p_back_f(C2PState& F, double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph) {
+  const DevEos& e = P.eos;
+  const bool ideal = e.kind == GRB_EOS_IDEAL_GAS;
+  C2POut& o = F.o;
+  WB& wb = F.wb;
+  if (F.ran) {
+    const uint32_t ret = F.ret;
+    if (ret & (SIG_EPS_HIGH | SIG_RHO_LOW | SIG_RHO_HIGH | SIG_VEL_HIGH)) o.floored = true;
+    if (ideal && (ret & SIG_EPS_LOW)) o.floored = true;
+    handle_sig(ret, F.lenient, o.err, o.fatal);
+  }
+  const bool excise = P.excise_by_radius ? (r_sph <= P.r_ex) : (m.alp <= P.alp_ex);
+  // which replacement of the primitives: 1 atmosphere, 2 temperature floor, 3 magnetisation
+  int rep = 0;
+  if (F.failed || excise || pr[GRB_P_RHO] < (1. + P.atmo_tol) * P.rho_fl) {
+    rep = 1;
+    o.floored = true;
+    o.err |= ERR_ALL_RESETS | ERR_ATMO;
+    pr[GRB_P_RHO] = P.rho_fl;
+    pr[GRB_P_YE] = P.ye_fl;
+    pr[GRB_P_TEMP] = P.temp_fl;
+    pr[GRB_P_ZX] = pr[GRB_P_ZY] = pr[GRB_P_ZZ] = 0.;
+    F.wb_ok = false;
+  } else if (pr[GRB_P_TEMP] < P.temp_fl) {
+    rep = 2;
+    pr[GRB_P_TEMP] = P.temp_fl;
+    o.err |= ERR_RESET_TAU | ERR_RESET_STILDE | ERR_RESET_ENTROPY | ERR_T_FLOORED;
+    if (ideal) o.floored = true;
+  } else {  // limit_primitives (c2p.cpp:63-115)
+    uint32_t s2 = 0;
+    const double z2max = P.max_w * P.max_w - 1.;
+    if (!F.wb_ok) { wb = wb_of(m, pr); F.wb_ok = true; }
+    if (wb.z2 >= z2max) {
+      s2 |= SIG_VEL_HIGH;
+      if (!kDry) {
+        const double zn = 0.99 * sqrt_f(z2max * rcp_f(wb.z2));
+        pr[GRB_P_ZX] *= zn; pr[GRB_P_ZY] *= zn; pr[GRB_P_ZZ] *= zn;
+        wb = wb_of(m, pr);
+      }
+    }
+    if (wb.b2 >= P.max_sigma * pr[GRB_P_RHO]) {
+      s2 |= SIG_SIGMA_HIGH;
+      rep = 3;
+      if (!kDry) pr[GRB_P_RHO] = 1.001 * wb.b2 / P.max_sigma;
+    }
+    handle_sig(s2, F.lenient, o.err, o.fatal);
+    if (s2) o.floored = true;
+  }
+  if (kDry) return;
+  if (rep) {
+    double cs2;
+    uint32_t q = 0;
+    pr[GRB_P_PRESS] = eos_PT(e, pr[GRB_P_EPS], cs2, nullptr, pr[GRB_P_TEMP], pr[GRB_P_RHO], q);
+    if (rep == 2) handle_eos_sig(q, F.lenient, o.err, o.fatal);
+    F.ent_ok = false;
+    pr[GRB_P_ENT] = ideal ? pr[GRB_P_EPS] : fmax(0.0, pr[GRB_P_TEMP] * e.igthm1);
+  }
+  if (!F.ent_ok) {
+    const double eth = pr[GRB_P_ENT];
+    pr[GRB_P_ENT] = ideal ? log(eth) * e.igm1 - log(pr[GRB_P_RHO])
+                          : log(fmax(eth, e.entropy_min)) * e.igthm1 - log(pr[GRB_P_RHO]);
+  }
+  if (!F.wb_ok) wb = wb_of(m, pr);
+  o.W = wb.W;
+  o.iW = wb.iW;
+  const uint32_t need = kAllCons ? ~0u : o.err;
+  const double D = pr[GRB_P_RHO] * wb.W;
+  c[0] = m.sqrtg * D;
+  c[6] = m.sqrtg * (pr[GRB_P_ENT] * D);
+  c[5] = c[0] * pr[GRB_P_YE];
+  if (need & (ERR_RESET_STILDE | ERR_RESET_TAU)) {
+    double zl[3], Bl[3];
+    mvs(m.g, pr + GRB_P_ZX, zl);
+    mvs(m.g, pr + GRB_P_BX, Bl);
+    const double rhoh = pr[GRB_P_RHO] * (1. + pr[GRB_P_EPS]) + pr[GRB_P_PRESS] + wb.b2;
+    const double pstar = pr[GRB_P_PRESS] + 0.5 * wb.b2;
+    const double hW = rhoh * wb.W;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      c[1 + i] = m.sqrtg * (hW * zl[i] - wb.Bz * ((Bl[i] + wb.Bz * zl[i]) * wb.iW));
+    c[4] = m.sqrtg * (hW * wb.W - pstar - wb.Bz * wb.Bz - D);
+  }
+}
+
+// The whole c2p in the tuned mode, and the FOFC flag's dry run.
+template <bool kAllCons = true>
+GRB_HD C2POut c2p_f(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph, double alp_bh_thresh) {
+  C2PState F = c2p_front_f<false>(c, pr, m, P, alp_bh_thresh);
+  if (F.backup) c2p_backup_f<false>(F, c, pr, m, P);
+  c2p_back_f<kAllCons>(F, c, pr, m, P, r_sph);
+  return F.o;
+}
+GRB_HD bool c2p_floored_f(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph) {
+  C2PState F = c2p_front_f<false, true>(c, pr, m, P, 1e30);
+  if (!F.done) c2p_back_f<true, true>(F, c, pr, m, P, r_sph);
   return F.o.floored;
 }
 

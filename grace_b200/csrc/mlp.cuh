@@ -305,6 +305,7 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
   return x ^ (x >> 31);
 }
 
+template <bool FAST = false>
 __device__ __forceinline__ Met batch_metric(const double* __restrict__ metric, int64_t n, int64_t t) {
   double g[6] = {1, 0, 0, 1, 0, 1}, b[3] = {0, 0, 0}, alp = 1.0;
   if (metric) {
@@ -314,7 +315,7 @@ __device__ __forceinline__ Met batch_metric(const double* __restrict__ metric, i
     for (int a = 0; a < 3; ++a) b[a] = metric[(6 + a) * n + t];
     alp = metric[9 * n + t];
   }
-  return make_met(g, b, alp);
+  return make_met<FAST>(g, b, alp);
 }
 
 // ---- batched c2p, plain or with the learned bracket ------------------------
@@ -340,8 +341,7 @@ __global__ void __launch_bounds__(256) k_mlp_pack(const float* __restrict__ P, M
 
 // One state per thread.  With the learned bracket every lane of a warp takes
 // part in the network (lanes past n with neutral inputs), then returns.
-// kFast: the tuned-mode c2p arithmetic (same functions up to rounding).
-template <bool kLearned, bool kFast = false>
+template <bool kLearned>
 __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch(DevParams P, int64_t n, const double* __restrict__ cons,
                                                           const double* __restrict__ metric,
                                                           double* __restrict__ prims, double* __restrict__ cons_out,
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch(DevParams P, int64_t 
       gs = mlp_bracket(S.net.nrm, out, mu0);
     }
     if (!active) return;
-    const C2POut o = c2p<kFast>(c, pr, m, P, 0.0, false, P.alp_bh_thresh, gs);
+    const C2POut o = c2p(c, pr, m, P, 0.0, false, P.alp_bh_thresh, gs);
     if (o.fatal) atomicOr(flags, o.fatal);
     pr[GRB_P_CS2] = 0.0;
 #pragma unroll
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch(DevParams P, int64_t 
   }
 }
 
-// ---- batched c2p with the entropy backup deferred ------------------------------
+// ---- batched c2p in the tuned mode: the entropy backup deferred ---------------
 // The states whose Kastaun result is distrusted (failed, eps too low, or
 // beta = 2P/b^2 <= beta_fallback) take the entropy-based backup solve.  In
 // a batch of mixed states nearly every warp holds some, so a one-pass
@@ -416,7 +416,7 @@ struct C2PDeferred {
   int64_t t;
 };
 
-template <bool kLearned, bool kFast>
+template <bool kLearned>
 __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, int64_t n,
                                                                 const double* __restrict__ cons,
                                                                 const double* __restrict__ metric,
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, in
   const int64_t t = (int64_t)blockIdx.x * kC2PThreads + threadIdx.x;
   const bool active = t < n;
   const int64_t ts = active ? t : 0;
-  const Met m = batch_metric(metric, n, ts);
+  const Met m = batch_metric<!kLearned>(metric, n, ts);
   double c[10], pr[13];
 #pragma unroll
   for (int v = 0; v < 10; ++v) c[v] = active ? cons[v * n + t] : 0.0;
@@ -456,7 +456,9 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, in
     gs = mlp_bracket(S.net.nrm, out, mu0);
   }
   C2PState F{};
-  if (active) F = c2p_front<kFast>(c, pr, m, P, false, P.alp_bh_thresh, gs);
+  if (active)
+    F = kLearned ? c2p_front<true>(c, pr, m, P, false, P.alp_bh_thresh, gs)
+                 : c2p_front_f<true>(c, pr, m, P, P.alp_bh_thresh);
   const bool later = active && !F.done && F.backup;
   // one slot per deferred lane, one atomic per warp
   const unsigned mask = __ballot_sync(0xffffffffu, later);
@@ -482,7 +484,7 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, in
     d.t = t;
     return;
   }
-  if (!F.done) c2p_back<kFast>(F, c, pr, m, P, 0.0);
+  if (!F.done) c2p_back_f(F, c, pr, m, P, 0.0);
   if (F.o.fatal) atomicOr(flags, F.o.fatal);
   pr[GRB_P_CS2] = 0.0;
 #pragma unroll
@@ -496,7 +498,6 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, in
 
 // The listed states: the entropy backup and the rest of the policy
 // (grid-stride over the count the front kernel left).
-template <bool kFast>
 __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_backup(DevParams P, int64_t n,
                                                                  const double* __restrict__ metric,
                                                                  double* __restrict__ prims,
@@ -514,9 +515,9 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_backup(DevParams P, i
     for (int v = 0; v < 13; ++v) pr[v] = d.pr[v];
     C2PState F = d.F;
     const int64_t t = d.t;
-    const Met m = batch_metric(metric, n, t);
-    c2p_backup(F, c, pr, m, P);
-    c2p_back<kFast>(F, c, pr, m, P, 0.0);
+    const Met m = batch_metric<true>(metric, n, t);
+    c2p_backup_f<true>(F, c, pr, m, P);
+    c2p_back_f(F, c, pr, m, P, 0.0);
     if (F.o.fatal) atomicOr(flags, F.o.fatal);
     pr[GRB_P_CS2] = 0.0;
 #pragma unroll

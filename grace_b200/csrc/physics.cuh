@@ -70,7 +70,7 @@ struct DevParams {
   int use_ent_backup;
   double rusanov_c_limit;
   int fofc, dmp_enable;
-  double dmp_M;
+  double dmp_M, idmp_M;  // idmp_M = 1 / dmp_M
   int recon, riemann, emf;
 };
 

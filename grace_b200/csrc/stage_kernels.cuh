@@ -540,7 +540,6 @@ __device__ __forceinline__ void fofc_flag_cell(const DevParams& P, const Geo& G,
   c[9] = 0.5 * (ct_bz(G, obz, B.emf, ix, i, j, k, q, dte) + ct_bz(G, obz, B.emf, ix, i, j, k + 1, q, dte));
   bool dmp = false;
   if (P.dmp_enable) {
-    const double invM = 1.0 / P.dmp_M;
     const int lv[2] = {GRB_DENS, GRB_TAU};
     for (int n = 0; n < 2 && !dmp; ++n) {
       double vmax = -1.7976931348623157e308, vmin = 1.7976931348623157e308;
@@ -548,18 +547,19 @@ __device__ __forceinline__ void fofc_flag_cell(const DevParams& P, const Geo& G,
         for (int jt = -1; jt <= 1; ++jt)
           for (int it = -1; it <= 1; ++it) {
             const double v = ns[cvar(G, i + it, j + jt, k + kt, lv[n], GRB_N_EVOL_VARS, q)];
-            vmax = fmax(vmax, v);
-            vmin = fmin(vmin, v);
+            vmax = v > vmax ? v : vmax;
+            vmin = v < vmin ? v : vmin;
           }
       const double t = c[lv[n]];
-      if (t > P.dmp_M * vmax || t < vmin * invM) dmp = true;
+      if (t > P.dmp_M * vmax || t < vmin * P.idmp_M) dmp = true;
     }
   }
   bool floored = false;
   if (!dmp) {  // the c2p dry run only matters when the DMP test passed
-    const Met m = cell_met(G, os, i, j, k, q);
+    const Met m = cell_met<kFast>(G, os, i, j, k, q);
     double pr[13];
-    floored = c2p_floored<kFast>(c, pr, m, P, cell_r(G, coords, ix, i, j, k, q));
+    const double r = cell_r(G, coords, ix, i, j, k, q);
+    floored = kFast ? c2p_floored_f(c, pr, m, P, r) : c2p_floored(c, pr, m, P, r);
   }
   if (floored || dmp) {
     int8_t* T = B.ftag;
@@ -958,48 +958,42 @@ __global__ void __launch_bounds__(128) k_dt(DevParams P, Geo G, Box box, const d
 // kDt: also the time-step reduction over the interior cells, from the
 // primitives just computed (the aux pass that ends an RK step).
 // One cell of the aux pass in three parts: aux_load (the cell's densitized
-// cons and cell-centred B, the metric, aux B), the c2p (in one piece, or
-// deferred at the entropy backup), aux_finish (prims, resets, C2P_ERR,
-// BDIV, the cell-centred E, the dt candidate of an interior cell (kDt) or
+// cons and cell-centred B, the metric; aux B and BDIV written), the c2p (in
+// one piece, or deferred at the entropy backup), aux_finish (prims, resets,
+// C2P_ERR, the cell-centred E, the dt candidate of an interior cell (kDt) or
 // +inf).
-struct AuxIn {
-  double c[10];
-  double bf[6];  // bx0, bx1, by0, by1, bz0, bz1
-};
-__device__ __forceinline__ Met aux_load(const DevParams& P, const Geo& G, int i, int j, int k, int64_t q,
-                                        const double* __restrict__ st, const double* __restrict__ bx,
-                                        const double* __restrict__ by, const double* __restrict__ bz,
-                                        double* __restrict__ aux, bool write_b, bool kFast, AuxIn& A) {
+template <bool kFast>
+__device__ __forceinline__ Met aux_load(const Geo& G, int i, int j, int k, int64_t q, const double* __restrict__ st,
+                                        const double* __restrict__ bx, const double* __restrict__ by,
+                                        const double* __restrict__ bz, double* __restrict__ aux,
+                                        const double* __restrict__ idx, bool write_b, double c[10]) {
   const int64_t c0 = cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
   const int64_t a0 = cvar(G, i, j, k, 0, GRB_N_AUX_VARS, q);
-  A.bf[0] = bx[bxi(G, i, j, k, q)]; A.bf[1] = bx[bxi(G, i + 1, j, k, q)];
-  A.bf[2] = by[byi(G, i, j, k, q)]; A.bf[3] = by[byi(G, i, j + 1, k, q)];
-  A.bf[4] = bz[bzi(G, i, j, k, q)]; A.bf[5] = bz[bzi(G, i, j, k + 1, q)];
+  const double b0 = bx[bxi(G, i, j, k, q)], b1 = bx[bxi(G, i + 1, j, k, q)];
+  const double b2 = by[byi(G, i, j, k, q)], b3 = by[byi(G, i, j + 1, k, q)];
+  const double b4 = bz[bzi(G, i, j, k, q)], b5 = bz[bzi(G, i, j, k + 1, q)];
 #pragma unroll
-  for (int v = 0; v < 7; ++v) A.c[v] = st[c0 + G.cells * v];
-  A.c[7] = 0.5 * (A.bf[0] + A.bf[1]);
-  A.c[8] = 0.5 * (A.bf[2] + A.bf[3]);
-  A.c[9] = 0.5 * (A.bf[4] + A.bf[5]);
-  const Met m = cell_met(G, st, i, j, k, q);
+  for (int v = 0; v < 7; ++v) c[v] = st[c0 + G.cells * v];
+  c[7] = 0.5 * (b0 + b1);
+  c[8] = 0.5 * (b2 + b3);
+  c[9] = 0.5 * (b4 + b5);
+  const Met m = cell_met<kFast>(G, st, i, j, k, q);
   if (write_b) {
-    const double isg = kFast ? 1.0 / m.sqrtg : 0.0;
-    aux[a0 + G.cells * GRB_BX] = kFast ? A.c[7] * isg : A.c[7] / m.sqrtg;
-    aux[a0 + G.cells * GRB_BY] = kFast ? A.c[8] * isg : A.c[8] / m.sqrtg;
-    aux[a0 + G.cells * GRB_BZ] = kFast ? A.c[9] * isg : A.c[9] / m.sqrtg;
+    const double dv = (b1 - b0) * idx[3 * q] + (b3 - b2) * idx[3 * q + 1] + (b5 - b4) * idx[3 * q + 2];
+    aux[a0 + G.cells * GRB_BX] = kFast ? c[7] * m.isqrtg : c[7] / m.sqrtg;
+    aux[a0 + G.cells * GRB_BY] = kFast ? c[8] * m.isqrtg : c[8] / m.sqrtg;
+    aux[a0 + G.cells * GRB_BZ] = kFast ? c[9] * m.isqrtg : c[9] / m.sqrtg;
+    aux[a0 + G.cells * GRB_BDIV] = kFast ? dv * m.isqrtg : dv / m.sqrtg;
   }
-  (void)P;
   return m;
 }
-// After the c2p: c, pr the c2p's output; A the cell's inputs (A.c its
-// cons before the c2p).
+// After the c2p: c, pr the c2p's output; cB the cell's densitized B.
 template <bool kDt, bool kFast>
 __device__ __forceinline__ double aux_finish(const DevParams& P, const Geo& G, int i, int j, int k, int64_t q,
-                                             double* __restrict__ st, double* __restrict__ aux,
-                                             const double* __restrict__ idx, const Met& m, const AuxIn& A,
-                                             const double c[10], const double pr[13], const C2POut& o,
-                                             const StageBufs& B, const DtArgs& dta) {
+                                             double* __restrict__ st, double* __restrict__ aux, const Met& m,
+                                             const double cB[3], const double c[10], const double pr[13],
+                                             const C2POut& o, const StageBufs& B, const DtArgs& dta) {
   double dtc = INFINITY;
-  const double ix[3] = {idx[3 * q], idx[3 * q + 1], idx[3 * q + 2]};
   const int64_t c0 = cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
   const int64_t a0 = cvar(G, i, j, k, 0, GRB_N_AUX_VARS, q);
   if (o.fatal) atomicOr(B.flags, o.fatal);
@@ -1013,7 +1007,7 @@ __device__ __forceinline__ double aux_finish(const DevParams& P, const Geo& G, i
   aux[a0 + G.cells * GRB_ZVECY] = pr[GRB_P_ZY];
   aux[a0 + G.cells * GRB_ZVECZ] = pr[GRB_P_ZZ];
   if (o.err & ERR_RESET_DENS) {
-    aux[a0 + G.cells * GRB_C2P_DENS_ERR] += A.c[GRB_DENS] - c[0];
+    aux[a0 + G.cells * GRB_C2P_DENS_ERR] += st[c0] - c[0];
     st[c0] = c[0];
   }
   if (o.err & ERR_RESET_STILDE)
@@ -1025,22 +1019,16 @@ __device__ __forceinline__ double aux_finish(const DevParams& P, const Geo& G, i
     const uint64_t prev = (uint64_t)aux[a0 + G.cells * GRB_C2P_ERR];
     aux[a0 + G.cells * GRB_C2P_ERR] = (double)(prev | (uint64_t)o.err);
   }
-  {
-    const double isg = kFast ? 1.0 / m.sqrtg : 0.0;
-    const double dv = (A.bf[1] - A.bf[0]) * ix[0] + (A.bf[3] - A.bf[2]) * ix[1] + (A.bf[5] - A.bf[4]) * ix[2];
-    aux[a0 + G.cells * GRB_BDIV] = kFast ? dv * isg : dv / m.sqrtg;
-  }
   if (P.emf == GRB_EMF_GS) {
-    const double cbx = A.c[7], cby = A.c[8], cbz = A.c[9];
     // tuned mode: 1/W of the final primitives from the c2p
     const double W = kFast ? o.W : sqrt(1. + sqs(m.g, pr + GRB_P_ZX));
     double vt[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a)
       vt[a] = (kFast ? m.alp * pr[GRB_P_ZX + a] * o.iW : m.alp * pr[GRB_P_ZX + a] / W) - m.beta[a];
-    B.ecenter[eci(G, i, j, k, 0, q)] = cby * vt[2] - cbz * vt[1];
-    B.ecenter[eci(G, i, j, k, 1, q)] = -cbx * vt[2] + cbz * vt[0];
-    B.ecenter[eci(G, i, j, k, 2, q)] = cbx * vt[1] - cby * vt[0];
+    B.ecenter[eci(G, i, j, k, 0, q)] = cB[1] * vt[2] - cB[2] * vt[1];
+    B.ecenter[eci(G, i, j, k, 1, q)] = -cB[0] * vt[2] + cB[2] * vt[0];
+    B.ecenter[eci(G, i, j, k, 2, q)] = cB[0] * vt[1] - cB[1] * vt[0];
   }
   if (kDt && i >= G.g && i < G.nx + G.g && j >= G.g && j < G.ny + G.g && k >= G.g && k < G.nz + G.g)
     dtc = dta.cfl / max_eigenspeed(P.eos, m, pr) * dta.dx[3 * q];
@@ -1054,16 +1042,13 @@ __device__ __forceinline__ double aux_cell(const DevParams& P, const Geo& G, int
                                            double* __restrict__ aux, const double* __restrict__ idx,
                                            const double* __restrict__ coords, const StageBufs& B,
                                            const DtArgs& dta) {
-  AuxIn A;
-  const Met m = aux_load(P, G, i, j, k, q, st, bx, by, bz, aux, true, kFast, A);
   double c[10], pr[13];
-#pragma unroll
-  for (int v = 0; v < 10; ++v) c[v] = A.c[v];
-  const double ix[3] = {idx[3 * q], idx[3 * q + 1], idx[3 * q + 2]};
-  const Guess none = no_guess();
-  const C2POut o =
-      c2p<kFast, !kFast>(c, pr, m, P, cell_r(G, coords, ix, i, j, k, q), false, P.alp_bh_thresh, none);
-  return aux_finish<kDt, kFast>(P, G, i, j, k, q, st, aux, idx, m, A, c, pr, o, B, dta);
+  const Met m = aux_load<kFast>(G, i, j, k, q, st, bx, by, bz, aux, idx, true, c);
+  const double cB[3] = {c[7], c[8], c[9]};
+  const double r = cell_r(G, coords, idx + 3 * q, i, j, k, q);
+  const C2POut o = kFast ? c2p_f<false>(c, pr, m, P, r, P.alp_bh_thresh)
+                         : c2p(c, pr, m, P, r, false, P.alp_bh_thresh, no_guess());
+  return aux_finish<kDt, kFast>(P, G, i, j, k, q, st, aux, m, cB, c, pr, o, B, dta);
 }
 
 // The aux pass with the entropy backups deferred (tuned candidate, for
@@ -1132,7 +1117,7 @@ __global__ void __launch_bounds__(128, MINB) k_aux_queue(DevParams P, Geo G, Box
   }
 }
 
-template <int MINB = 1, bool kDt = false, bool kFast = false>
+template <int MINB = 1, bool kDt = false>
 __global__ void __launch_bounds__(128, MINB) k_aux_front(DevParams P, Geo G, Box box, double* __restrict__ st,
                                                     const double* __restrict__ bx,
                                                     const double* __restrict__ by,
@@ -1145,20 +1130,18 @@ __global__ void __launch_bounds__(128, MINB) k_aux_front(DevParams P, Geo G, Box
   int64_t q = 0;
   double dtc = INFINITY;
   const bool active = decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q);
-  AuxIn A;
   Met m;
-  double c[10], pr[13];
+  double c[10], pr[13], cB[3];
   C2PState F{};
   double r = 0.0;
   if (active) {
-    m = aux_load(P, G, i, j, k, q, st, bx, by, bz, aux, true, kFast, A);
+    m = aux_load<true>(G, i, j, k, q, st, bx, by, bz, aux, idx, true, c);
 #pragma unroll
-    for (int v = 0; v < 10; ++v) c[v] = A.c[v];
-    const double ix[3] = {idx[3 * q], idx[3 * q + 1], idx[3 * q + 2]};
-    r = cell_r(G, coords, ix, i, j, k, q);
-    F = c2p_front<kFast>(c, pr, m, P, false, P.alp_bh_thresh, no_guess());
+    for (int a = 0; a < 3; ++a) cB[a] = c[7 + a];
+    r = cell_r(G, coords, idx + 3 * q, i, j, k, q);
+    F = c2p_front_f<false>(c, pr, m, P, P.alp_bh_thresh);
   }
-  const bool later = active && !F.done && F.backup;
+  const bool later = active && F.backup;
   const unsigned mask = __ballot_sync(0xffffffffu, later);
   unsigned long long base = 0;
   const int lane = threadIdx.x & 31;
@@ -1175,16 +1158,14 @@ __global__ void __launch_bounds__(128, MINB) k_aux_front(DevParams P, Geo G, Box
       d.F = F;
       d.i = i; d.j = j; d.k = k; d.q = q;
     } else {
-      if (!F.done) {
-        if (F.backup) c2p_backup(F, c, pr, m, P);
-        c2p_back<kFast, !kFast>(F, c, pr, m, P, r);
-      }
-      dtc = aux_finish<kDt, kFast>(P, G, i, j, k, q, st, aux, idx, m, A, c, pr, F.o, B, dta);
+      if (F.backup) c2p_backup_f<false>(F, c, pr, m, P);
+      c2p_back_f<false>(F, c, pr, m, P, r);
+      dtc = aux_finish<kDt, true>(P, G, i, j, k, q, st, aux, m, cB, c, pr, F.o, B, dta);
     }
   }
   if (kDt) dt_reduce(dtc, dta.out);
 }
-template <int MINB = 1, bool kDt = false, bool kFast = false>
+template <int MINB = 1, bool kDt = false>
 __global__ void __launch_bounds__(128, MINB) k_aux_backup(DevParams P, Geo G, double* __restrict__ st,
                                                      const double* __restrict__ bx,
                                                      const double* __restrict__ by,
@@ -1199,18 +1180,17 @@ __global__ void __launch_bounds__(128, MINB) k_aux_backup(DevParams P, Geo G, do
     const AuxDeferred& d = static_cast<const AuxDeferred*>(B.adefer)[e];
     const int i = d.i, j = d.j, k = d.k;
     const int64_t q = d.q;
-    AuxIn A;
-    const Met m = aux_load(P, G, i, j, k, q, st, bx, by, bz, aux, false, kFast, A);
     double c[10], pr[13];
+    const Met m = aux_load<true>(G, i, j, k, q, st, bx, by, bz, aux, idx, false, c);
+    const double cB[3] = {c[7], c[8], c[9]};
 #pragma unroll
     for (int v = 0; v < 10; ++v) c[v] = d.c[v];
 #pragma unroll
     for (int v = 0; v < 13; ++v) pr[v] = d.pr[v];
     C2PState F = d.F;
-    const double ix[3] = {idx[3 * q], idx[3 * q + 1], idx[3 * q + 2]};
-    c2p_backup(F, c, pr, m, P);
-    c2p_back<kFast, !kFast>(F, c, pr, m, P, cell_r(G, coords, ix, i, j, k, q));
-    dtc = fmin(dtc, aux_finish<kDt, kFast>(P, G, i, j, k, q, st, aux, idx, m, A, c, pr, F.o, B, dta));
+    c2p_backup_f<false>(F, c, pr, m, P);
+    c2p_back_f<false>(F, c, pr, m, P, cell_r(G, coords, idx + 3 * q, i, j, k, q));
+    dtc = fmin(dtc, aux_finish<kDt, true>(P, G, i, j, k, q, st, aux, m, cB, c, pr, F.o, B, dta));
   }
   if (kDt) dt_reduce(dtc, dta.out);
 }
