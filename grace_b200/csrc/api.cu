@@ -445,14 +445,14 @@ void launch_update_tuned(int v, unsigned nb, cudaStream_t s, const DevParams& P,
   if (v >= 3) v -= 3;
   if (md) {
     static_assert(kMinBCached[1] == 3 && kMinBCached[2] == 4, "update candidates");
-    if (v == 1) k_update<3, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B, md);
-    else if (v == 2) k_update<4, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B, md);
-    else k_update<1, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B, md);
+    if (v == 1) k_update<3, true, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B, md);
+    else if (v == 2) k_update<4, true, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B, md);
+    else k_update<1, true, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B, md);
     return;
   }
-  if (v == 1) k_update<4><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B);
-  else if (v == 2) k_update<5><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B);
-  else k_update<1><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B);
+  if (v == 1) k_update<4, false, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B);
+  else if (v == 2) k_update<5, false, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B);
+  else k_update<1, false, true><<<nb, 128, 0, s>>>(P, G, b, dt, dtfact, ns, os, aux, idx, B);
 }
 // Work-queue aux pass: one wave of CTAs (occupancy x SMs) pulling tiles.
 template <int MINB, bool kDt>
@@ -706,7 +706,7 @@ int stage_tuned(grb_handle* h, const Geo& G, const grb_grid* g, double dt, doubl
   {
     KScope ks(h, s, GRB_KIND_EMF);
     if (P.emf == GRB_EMF_GS) k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B);
-    else k_emf_uct<<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, old->bx, old->by, old->bz, B);
+    else k_emf_uct<true><<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, old->bx, old->by, old->bz, B);
     ++launches;
   }
   if (P.fofc && P.emf == GRB_EMF_GS) {
@@ -978,7 +978,7 @@ int grb_advance_substep(grb_handle* h, const grb_grid* g, double t, double dt, d
   if (P.emf == GRB_EMF_GS)
     k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B);
   else
-    k_emf_uct<<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, old->bx, old->by, old->bz, B);
+    k_emf_uct<false><<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, old->bx, old->by, old->bz, B);
   ++h->launches;
   }
   if (P.fofc && P.emf == GRB_EMF_GS) {
@@ -2527,7 +2527,7 @@ extern "C" int grb_advance_substep_static(const grb_params* p, const grb_grid* g
     if (P.emf == GRB_EMF_GS)
       k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B);
     else
-      k_emf_uct<<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, obx, oby, obz, B);
+      k_emf_uct<false><<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, obx, oby, obz, B);
     if (P.fofc && P.emf == GRB_EMF_GS) {
       if (cudaMemsetAsync(B.ftag, 0, L.ftag * nq, s) != cudaSuccess) return GRB_ERR_CUDA;
       if (cudaMemsetAsync(B.etag, 0, L.etag * nq, s) != cudaSuccess) return GRB_ERR_CUDA;

@@ -436,21 +436,42 @@ GRB_HD ConsFlux cons_flux(double alp, const double beta[3], const double g[6], d
 // geometric sources (grmhd_subexpressions.hh:158-292)
 //   S_tau = alpha [ (T00 b^i b^j + 2 T0i b^j + Tij) K_ij - (T00 b^i + T0i) d_i alpha ]
 //   S_Sj  = alpha [ 1/2 T00 d_j g00 + T0i d_j g0i + 1/2 Tik d_j g_ik ]
-GRB_HD void geom_sources(const Met& m, const double K[6], const double dalp[3],
-                         const double dg[18], const double db[9], double rho, double press,
-                         double eps, const double B[3], const double z[3], double W,
-                         double& stau, double sS[3]) {
+// der(jd, dalp, db, dg): the derivatives along jd of alpha, beta^c and g_c; one
+// direction's ten are live at a time.  FAST (tuned mode): b^mu, u^mu and W
+// from 1/alpha and 1/W (rsqrt_f) instead of a dozen quotients, equal up to
+// rounding.
+template <bool FAST, class Der>
+GRB_HD void geom_sources(const Met& m, const double K[6], Der&& der, double rho, double press, double eps,
+                         const double B[3], const double z[3], double& stau, double sS[3]) {
   const double alp = m.alp;
   const double* beta = m.beta;
-  double b[4], b2;
-  comoving_b(alp, beta, m.g, B, z, W, b, b2);
+  double b[4], b2, u0, u[3], ia2;
+  if (FAST) {
+    double zl[3];
+    mvs(m.g, z, zl);
+    const double q = 1. + (z[0] * zl[0] + z[1] * zl[1] + z[2] * zl[2]);
+    const double iW = rsqrt_f(q);
+    const double Bz = B[0] * zl[0] + B[1] * zl[1] + B[2] * zl[2];
+    u0 = q * iW * m.ialp;
+    b[0] = Bz * m.ialp;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      u[i] = z[i] - u0 * beta[i];
+      b[i + 1] = (B[i] + Bz * u[i]) * iW;
+    }
+    b2 = (sqs(m.g, B) + Bz * Bz) * (iW * iW);
+    ia2 = m.ialp * m.ialp;
+  } else {
+    const double W = lorentz(m.g, z);
+    comoving_b(alp, beta, m.g, B, z, W, b, b2);
+    ia2 = 1. / (alp * alp);
+    u0 = W / alp;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) u[i] = z[i] - W * beta[i] / alp;
+  }
   const double rhoh = rho * (1. + eps) + press + b2;
   const double pstar = press + 0.5 * b2;
-  const double ia2 = 1. / (alp * alp);
-  const double u0 = W / alp;
-  double u[3], T0[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) u[i] = z[i] - W * beta[i] / alp;
+  double T0[3];
   const double T00 = rhoh * u0 * u0 - pstar * ia2 - b[0] * b[0];
 #pragma unroll
   for (int i = 0; i < 3; ++i) T0[i] = rhoh * u0 * u[i] + pstar * beta[i] * ia2 - b[0] * b[i + 1];
@@ -469,20 +490,18 @@ GRB_HD void geom_sources(const Met& m, const double K[6], const double dalp[3],
     kt += w * (T00 * beta[i] * beta[j] + T0[i] * beta[j] + T0[j] * beta[i] + T[a]) * K[a];
   }
   double at = 0.;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) at += (T00 * beta[i] + T0[i]) * dalp[i];
-  stau = alp * (kt - at);
   double betal[3];
   mvs(m.g, beta, betal);
 #pragma unroll
   for (int jd = 0; jd < 3; ++jd) {
-    const double* dgj = dg + 6 * jd;
-    const double* dbj = db + 3 * jd;
+    double dalp, dbj[3], dgj[6];
+    der(jd, dalp, dbj, dgj);
+    at += (T00 * beta[jd] + T0[jd]) * dalp;
     double dbv[3];  // beta^k d_j g_ik
     mvs(dgj, beta, dbv);
     double gdb[3];  // g_ik d_j beta^k
     mvs(m.g, dbj, gdb);
-    const double dg00 = -2. * alp * dalp[jd] + (beta[0] * dbv[0] + beta[1] * dbv[1] + beta[2] * dbv[2]) +
+    const double dg00 = -2. * alp * dalp + (beta[0] * dbv[0] + beta[1] * dbv[1] + beta[2] * dbv[2]) +
                         2. * (betal[0] * dbj[0] + betal[1] * dbj[1] + betal[2] * dbj[2]);
     double acc = 0.5 * T00 * dg00;
 #pragma unroll
@@ -494,6 +513,7 @@ GRB_HD void geom_sources(const Met& m, const double K[6], const double dalp[3],
     }
     sS[jd] = alp * acc;
   }
+  stau = alp * (kt - at);
 }
 
 GRB_HD double hll(double fL, double fR, double uL, double uR, double cmin, double cmax) {

@@ -380,12 +380,18 @@ __global__ void __launch_bounds__(128) k_emf_gs(Geo G, Box box, StageBufs B) {
 }
 
 // ---- UCT edge EMF (evolve.cpp:1131-1340) ----------------------------------
+template <bool FAST>
 __device__ __forceinline__ void recon_line(int recon, const double* p, int64_t s, double& L, double& R) {
   double u[6];
 #pragma unroll
   for (int o = 0; o < 6; ++o) u[o] = __ldg(p + (o - 3) * s);
-  recon6(recon, u, L, R);
+  if (FAST) recon6_fast(recon, u, L, R);
+  else recon6(recon, u, L, R);
 }
+// FAST (tuned mode): the reconstructions by weno_z_face (one reciprocal a
+// state where weno_z takes four quotients; twelve lines a cell), the HLL
+// quotients by rcp_f.
+template <bool FAST>
 __global__ void __launch_bounds__(128) k_emf_uct(DevParams P, Geo G, Box box,
                                                   const double* __restrict__ bx,
                                                   const double* __restrict__ by,
@@ -394,6 +400,9 @@ __global__ void __launch_bounds__(128) k_emf_uct(DevParams P, Geo G, Box box,
   int64_t q;
   if (!decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q)) return;
   const int rk = P.recon;
+  auto hll = [](double fL, double fR, double uL, double uR, double cn, double cx) {
+    return FAST ? (cx * fL + cn * fR - cx * cn * (uR - uL)) * rcp_f(cx + cn) : grb::hll(fL, fR, uL, uR, cn, cx);
+  };
   const double* VB = B.vbar;
   // strides of the three face arrays along x, y, z
   const int64_t sxx = 1, sxy = G.NX + 1, sxz = (int64_t)(G.NX + 1) * G.NY;
@@ -402,10 +411,10 @@ __global__ void __launch_bounds__(128) k_emf_uct(DevParams P, Geo G, Box box,
   const int64_t vs[3] = {1, G.FX, (int64_t)G.FX * G.FY};
   if (i < G.nx + G.g) {  // E^x at (i, j-1/2, k-1/2)
     double ByL, ByR, vzL, vzR, BzL, BzR, vyL, vyR;
-    recon_line(rk, by + byi(G, i, j, k, q), syz, ByL, ByR);
-    recon_line(rk, VB + vbi(G, i, j, k, 1, 1, q), vs[2], vzL, vzR);
-    recon_line(rk, bz + bzi(G, i, j, k, q), szy, BzL, BzR);
-    recon_line(rk, VB + vbi(G, i, j, k, 1, 2, q), vs[1], vyL, vyR);
+    recon_line<FAST>(rk, by + byi(G, i, j, k, q), syz, ByL, ByR);
+    recon_line<FAST>(rk, VB + vbi(G, i, j, k, 1, 1, q), vs[2], vzL, vzR);
+    recon_line<FAST>(rk, bz + bzi(G, i, j, k, q), szy, BzL, BzR);
+    recon_line<FAST>(rk, VB + vbi(G, i, j, k, 1, 2, q), vs[1], vyL, vyR);
     const double cmin_y = fmax(VB[vbi(G, i, j, k, 2, 1, q)], VB[vbi(G, i, j, k - 1, 2, 1, q)]);
     const double cmax_y = fmax(VB[vbi(G, i, j, k, 3, 1, q)], VB[vbi(G, i, j, k - 1, 3, 1, q)]);
     const double cmin_z = fmax(VB[vbi(G, i, j, k, 2, 2, q)], VB[vbi(G, i, j - 1, k, 2, 2, q)]);
@@ -415,10 +424,10 @@ __global__ void __launch_bounds__(128) k_emf_uct(DevParams P, Geo G, Box box,
   }
   if (j < G.ny + G.g) {  // E^y at (i-1/2, j, k-1/2)
     double BzL, BzR, vxL, vxR, BxL, BxR, vzL, vzR;
-    recon_line(rk, bz + bzi(G, i, j, k, q), szx, BzL, BzR);
-    recon_line(rk, VB + vbi(G, i, j, k, 0, 2, q), vs[0], vxL, vxR);
-    recon_line(rk, bx + bxi(G, i, j, k, q), sxz, BxL, BxR);
-    recon_line(rk, VB + vbi(G, i, j, k, 1, 0, q), vs[2], vzL, vzR);
+    recon_line<FAST>(rk, bz + bzi(G, i, j, k, q), szx, BzL, BzR);
+    recon_line<FAST>(rk, VB + vbi(G, i, j, k, 0, 2, q), vs[0], vxL, vxR);
+    recon_line<FAST>(rk, bx + bxi(G, i, j, k, q), sxz, BxL, BxR);
+    recon_line<FAST>(rk, VB + vbi(G, i, j, k, 1, 0, q), vs[2], vzL, vzR);
     const double cmin_z = fmax(VB[vbi(G, i, j, k, 2, 2, q)], VB[vbi(G, i - 1, j, k, 2, 2, q)]);
     const double cmax_z = fmax(VB[vbi(G, i, j, k, 3, 2, q)], VB[vbi(G, i - 1, j, k, 3, 2, q)]);
     const double cmin_x = fmax(VB[vbi(G, i, j, k, 2, 0, q)], VB[vbi(G, i, j, k - 1, 2, 0, q)]);
@@ -428,10 +437,10 @@ __global__ void __launch_bounds__(128) k_emf_uct(DevParams P, Geo G, Box box,
   }
   if (k < G.nz + G.g) {  // E^z at (i-1/2, j-1/2, k)
     double BxL, BxR, vyL, vyR, ByL, ByR, vxL, vxR;
-    recon_line(rk, bx + bxi(G, i, j, k, q), sxy, BxL, BxR);
-    recon_line(rk, VB + vbi(G, i, j, k, 0, 0, q), vs[1], vyL, vyR);
-    recon_line(rk, by + byi(G, i, j, k, q), syx, ByL, ByR);
-    recon_line(rk, VB + vbi(G, i, j, k, 0, 1, q), vs[0], vxL, vxR);
+    recon_line<FAST>(rk, bx + bxi(G, i, j, k, q), sxy, BxL, BxR);
+    recon_line<FAST>(rk, VB + vbi(G, i, j, k, 0, 0, q), vs[1], vyL, vyR);
+    recon_line<FAST>(rk, by + byi(G, i, j, k, q), syx, ByL, ByR);
+    recon_line<FAST>(rk, VB + vbi(G, i, j, k, 0, 1, q), vs[0], vxL, vxR);
     const double cmin_x = fmax(VB[vbi(G, i, j, k, 2, 0, q)], VB[vbi(G, i, j - 1, k, 2, 0, q)]);
     const double cmax_x = fmax(VB[vbi(G, i, j, k, 3, 0, q)], VB[vbi(G, i, j - 1, k, 3, 0, q)]);
     const double cmin_y = fmax(VB[vbi(G, i, j, k, 2, 1, q)], VB[vbi(G, i - 1, j, k, 2, 1, q)]);
@@ -526,14 +535,15 @@ __device__ __forceinline__ void fofc_flag_cell(const DevParams& P, const Geo& G,
                                                const double* __restrict__ coords, const StageBufs& B) {
   const double ix[3] = {idx[3 * q], idx[3 * q + 1], idx[3 * q + 2]};
   double c[10];
-  const double* F = B.flux;
+  const double* F = B.flux + flx(G, i, j, k, 0, 0, q);
+  const double* u = ns + cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
+  const int64_t fy = 7 * G.fcells, fz = 14 * G.fcells, sy = G.FX, sz = (int64_t)G.FX * G.FY;
 #pragma unroll
-  for (int v = 0; v < 7; ++v)
-    c[v] = ns[cvar(G, i, j, k, v, GRB_N_EVOL_VARS, q)] +
-           dt * dtfact *
-               ((F[flx(G, i, j, k, v, 0, q)] - F[flx(G, i + 1, j, k, v, 0, q)]) * ix[0] +
-                (F[flx(G, i, j, k, v, 1, q)] - F[flx(G, i, j + 1, k, v, 1, q)]) * ix[1] +
-                (F[flx(G, i, j, k, v, 2, q)] - F[flx(G, i, j, k + 1, v, 2, q)]) * ix[2]);
+  for (int v = 0; v < 7; ++v) {
+    const double* f = F + G.fcells * v;
+    c[v] = u[G.cells * v] + dt * dtfact *
+                                ((f[0] - f[1]) * ix[0] + (f[fy] - f[fy + sy]) * ix[1] + (f[fz] - f[fz + sz]) * ix[2]);
+  }
   const double dte = dt * dtfact;
   c[7] = 0.5 * (ct_bx(G, obx, B.emf, ix, i, j, k, q, dte) + ct_bx(G, obx, B.emf, ix, i + 1, j, k, q, dte));
   c[8] = 0.5 * (ct_by(G, oby, B.emf, ix, i, j, k, q, dte) + ct_by(G, oby, B.emf, ix, i, j + 1, k, q, dte));
@@ -546,7 +556,7 @@ __device__ __forceinline__ void fofc_flag_cell(const DevParams& P, const Geo& G,
       for (int kt = -1; kt <= 1; ++kt)
         for (int jt = -1; jt <= 1; ++jt)
           for (int it = -1; it <= 1; ++it) {
-            const double v = ns[cvar(G, i + it, j + jt, k + kt, lv[n], GRB_N_EVOL_VARS, q)];
+            const double v = u[G.cells * lv[n] + it + (int64_t)G.NX * (jt + G.NY * kt)];
             vmax = v > vmax ? v : vmax;
             vmin = v < vmin ? v : vmin;
           }
@@ -755,33 +765,26 @@ __global__ void __launch_bounds__(128) k_fofc_edges(Geo G, Box box, StageBufs B)
 }
 
 // ---- flux divergence + geometric sources on interior cells -----------------
-// Sixth-order centred derivatives of the lapse, shift and 3-metric at one
-// cell (os + c0: the cell's variable 0), one spacing h for all axes as in
-// grmhd.hh:232-235: dalp[jd], db[3 jd + c] = d_jd beta^c,
-// dg[6 jd + c] = d_jd g_c.  The 30 values in this order are also the
-// layout of the static-metric cache (kMetDer doubles per cell).
+// Sixth-order centred derivatives along jd (stride s) of the lapse, shift and
+// 3-metric at one cell (os + c0: the cell's variable 0), one spacing h for all
+// axes as in grmhd.hh:232-235.  The static-metric cache holds the 30 values
+// of the three directions (kMetDer doubles per cell): d_jd alpha in
+// [jd], d_jd beta^c in [3 + 3 jd + c], d_jd g_c in [12 + 6 jd + c].
 constexpr int kMetDer = 30;
-__device__ __forceinline__ void metric_derivs(const Geo& G, const double* __restrict__ os, int64_t c0, double h,
-                                              double dalp[3], double db[9], double dg[18]) {
-  const int64_t sy = G.NX, sz = (int64_t)G.NX * G.NY;
-  auto der = [&](int v, double o[3]) {
+__device__ __forceinline__ void metric_derivs(const Geo& G, const double* __restrict__ os, int64_t c0, int64_t s,
+                                              double h, double& dalp, double db[3], double dg[6]) {
+  auto der = [&](int v) {
     const double* p = os + c0 + G.cells * v;
-    o[0] = fd6(p[-3], p[-2], p[-1], p[1], p[2], p[3], h);
-    o[1] = fd6(p[-3 * sy], p[-2 * sy], p[-sy], p[sy], p[2 * sy], p[3 * sy], h);
-    o[2] = fd6(p[-3 * sz], p[-2 * sz], p[-sz], p[sz], p[2 * sz], p[3 * sz], h);
+    return fd6(p[-3 * s], p[-2 * s], p[-s], p[s], p[2 * s], p[3 * s], h);
   };
-  double t3[3];
-  der(GRB_ALP, dalp);
+  dalp = der(GRB_ALP);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    der(GRB_BETAX + c, t3);
-    db[c] = t3[0]; db[3 + c] = t3[1]; db[6 + c] = t3[2];
-  }
+  for (int c = 0; c < 3; ++c) db[c] = der(GRB_BETAX + c);
 #pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    der(GRB_GXX + c, t3);
-    dg[c] = t3[0]; dg[6 + c] = t3[1]; dg[12 + c] = t3[2];
-  }
+  for (int c = 0; c < 6; ++c) dg[c] = der(GRB_GXX + c);
+}
+__device__ __forceinline__ int64_t axis_stride(const Geo& G, int jd) {
+  return jd == 0 ? 1 : jd == 1 ? (int64_t)G.NX : (int64_t)G.NX * G.NY;
 }
 // Offset of derivative d of interior cell (i, j, k) of block q in the
 // static-metric cache: [q][d][k - g][j - g][i - g].
@@ -794,58 +797,74 @@ __global__ void __launch_bounds__(128) k_metric_derivs(Geo G, Box box, const dou
   int i, j, k;
   int64_t q;
   if (!decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q)) return;
-  double d[kMetDer];
-  metric_derivs(G, os, cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q), idx[3 * q], d, d + 3, d + 12);
 #pragma unroll
-  for (int c = 0; c < kMetDer; ++c) md[mdi(G, i, j, k, c, q)] = d[c];
+  for (int jd = 0; jd < 3; ++jd) {
+    double a, b[3], g[6];
+    metric_derivs(G, os, cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q), axis_stride(G, jd), idx[3 * q], a, b, g);
+    md[mdi(G, i, j, k, jd, q)] = a;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) md[mdi(G, i, j, k, 3 + 3 * jd + c, q)] = b[c];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) md[mdi(G, i, j, k, 12 + 6 * jd + c, q)] = g[c];
+  }
 }
 
 // add_fluxes_and_source_terms for one interior cell.  kCached: the metric
 // derivatives from the static-metric cache md (tuned mode, Cowling) instead
-// of differentiating the metric here.
-template <bool kCached>
+// of differentiating the metric here.  kFast: the tuned mode's arithmetic.
+// Memory bound (about 110 doubles a cell with the cache): what counts is
+// loads in flight, so the sources take the derivatives direction by direction
+// (10 live instead of 30) and the registers go to occupancy.
+template <bool kCached, bool kFast>
 __device__ __forceinline__ void update_cell(const DevParams& P, const Geo& G, int i, int j, int k, int64_t q,
                                             double dt, double dtfact, double* __restrict__ ns,
                                             const double* __restrict__ os, const double* __restrict__ aux,
                                             const double* __restrict__ idx, const StageBufs& B,
                                             const double* __restrict__ md) {
   const double ix[3] = {idx[3 * q], idx[3 * q + 1], idx[3 * q + 2]};
-  const Met m = cell_met(G, os, i, j, k, q);
-  const int64_t a0 = cvar(G, i, j, k, 0, GRB_N_AUX_VARS, q);
-  const double z[3] = {aux[a0 + G.cells * GRB_ZVECX], aux[a0 + G.cells * GRB_ZVECY], aux[a0 + G.cells * GRB_ZVECZ]};
-  const double Bv[3] = {aux[a0 + G.cells * GRB_BX], aux[a0 + G.cells * GRB_BY], aux[a0 + G.cells * GRB_BZ]};
-  const double W = lorentz(m.g, z);
+  const Met m = cell_met<kFast>(G, os, i, j, k, q);
+  const double* a = aux + cvar(G, i, j, k, 0, GRB_N_AUX_VARS, q);
+  const double z[3] = {a[G.cells * GRB_ZVECX], a[G.cells * GRB_ZVECY], a[G.cells * GRB_ZVECZ]};
+  const double Bv[3] = {a[G.cells * GRB_BX], a[G.cells * GRB_BY], a[G.cells * GRB_BZ]};
   const int64_t c0 = cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
-  double d[kMetDer];
-  if (kCached) {
-    const int64_t m0 = mdi(G, i, j, k, 0, q), ms = (int64_t)G.nx * G.ny * G.nz;
-#pragma unroll
-    for (int c = 0; c < kMetDer; ++c) d[c] = md[m0 + c * ms];
-  } else {
-    metric_derivs(G, os, c0, ix[0], d, d + 3, d + 12);
-  }
   double K[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) K[c] = os[c0 + G.cells * (GRB_KXX + c)];
   double stau, sS[3];
-  geom_sources(m, K, d, d + 12, d + 3, aux[a0 + G.cells * GRB_RHO], aux[a0 + G.cells * GRB_PRESS],
-               aux[a0 + G.cells * GRB_EPS], Bv, z, W, stau, sS);
-  const double* F = B.flux;
+  geom_sources<kFast>(
+      m, K,
+      [&](int jd, double& dalp, double db[3], double dg[6]) {
+        if (kCached) {
+          const int64_t ms = (int64_t)G.nx * G.ny * G.nz;
+          const double* p = md + mdi(G, i, j, k, 0, q);
+          dalp = p[jd * ms];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) db[c] = p[(3 + 3 * jd + c) * ms];
+#pragma unroll
+          for (int c = 0; c < 6; ++c) dg[c] = p[(12 + 6 * jd + c) * ms];
+        } else {
+          metric_derivs(G, os, c0, axis_stride(G, jd), ix[0], dalp, db, dg);
+        }
+      },
+      a[G.cells * GRB_RHO], a[G.cells * GRB_PRESS], a[G.cells * GRB_EPS], Bv, z, stau, sS);
+  const double* F = B.flux + flx(G, i, j, k, 0, 0, q);
+  const int64_t fy = 7 * G.fcells, fz = 14 * G.fcells, sy = G.FX, sz = (int64_t)G.FX * G.FY;
   const double sd = m.sqrtg * dt * dtfact;
   double src[7] = {0., sd * sS[0], sd * sS[1], sd * sS[2], sd * stau, 0., 0.};
 #pragma unroll
   for (int v = 0; v < GRB_N_HRSC; ++v) {
     double* p = ns + c0 + G.cells * v;
+    const double* f = F + G.fcells * v;
     double u = *p;
     if (v >= 1 && v <= 4) u += src[v];
-    const double dFx = (F[flx(G, i, j, k, v, 0, q)] - F[flx(G, i + 1, j, k, v, 0, q)]) * ix[0];
-    const double dFy = (F[flx(G, i, j, k, v, 1, q)] - F[flx(G, i, j + 1, k, v, 1, q)]) * ix[1];
-    const double dFz = (F[flx(G, i, j, k, v, 2, q)] - F[flx(G, i, j, k + 1, v, 2, q)]) * ix[2];
+    const double dFx = (f[0] - f[1]) * ix[0];
+    const double dFy = (f[fy] - f[fy + sy]) * ix[1];
+    const double dFz = (f[fz] - f[fz + sz]) * ix[2];
     *p = u + dt * dtfact * ((dFx + dFy) + dFz);
   }
 }
 
-template <int MINB = 1, bool kCached = false>
+template <int MINB = 1, bool kCached = false, bool kFast = false>
 __global__ void __launch_bounds__(128, MINB) k_update(DevParams P, Geo G, Box box, double dt, double dtfact,
                                                  double* __restrict__ ns, const double* __restrict__ os,
                                                  const double* __restrict__ aux,
@@ -854,7 +873,7 @@ __global__ void __launch_bounds__(128, MINB) k_update(DevParams P, Geo G, Box bo
   int i, j, k;
   int64_t q;
   if (!decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q)) return;
-  update_cell<kCached>(P, G, i, j, k, q, dt, dtfact, ns, os, aux, idx, B, md);
+  update_cell<kCached, kFast>(P, G, i, j, k, q, dt, dtfact, ns, os, aux, idx, B, md);
 }
 
 // k_update as a persistent launch (tuned candidate); per cell the same work.
@@ -867,7 +886,7 @@ __global__ void __launch_bounds__(128, MINB) k_update_queue(DevParams P, Geo G, 
                                                        const double* __restrict__ md,
                                                        unsigned long long* __restrict__ queue) {
   for_queue_items(box, queue, [&](int i, int j, int k, int64_t q) {
-    update_cell<kCached>(P, G, i, j, k, q, dt, dtfact, ns, os, aux, idx, B, md);
+    update_cell<kCached, true>(P, G, i, j, k, q, dt, dtfact, ns, os, aux, idx, B, md);
   });
 }
 
