@@ -221,6 +221,10 @@ constexpr int kMinBC2p[3] = {3, 4, 5};
 // The update kernel that reads the static-metric cache: 1, 3, 4.
 constexpr int kMinBCached[3] = {1, 3, 4};
 constexpr int kNumVar = 3;
+// The plain mode's kernels: 4 CTAs of 128 threads per SM (128 registers).
+// Uncapped they take 160 to 254 and hold 2 or 3 CTAs, too few to cover the
+// latency of their dependent FP64 chains.
+constexpr int kPlainMinB = 4;
 
 // ---- TMA-staged flux kernel: tensor maps and tile geometry ----------------
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no -lcuda).
@@ -676,6 +680,21 @@ static unsigned fofc_list_grid() {
   return (unsigned)(3 * sms[dev]);
 }
 
+// The faces of direction dir that a stage reads: [g-1, n+g+2) along it;
+// across, one row of cells beyond the interior for the Gardiner-Stone edges
+// and the FOFC cells, three for the UCT reconstructions.  The reference
+// computes the whole transverse ghost range (evolve.cpp:908-922): for 16^3
+// blocks 1.8 times as many faces, whose values nothing reads.
+Box face_box(const Geo& G, int emf, int dir, int64_t nq) {
+  const int nn[3] = {G.nx, G.ny, G.nz}, w = emf == GRB_EMF_GS ? 1 : 3;
+  int lo[3], n[3];
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = G.g - (a == dir ? 1 : w);
+    n[a] = nn[a] + (a == dir ? 3 : 2 * w);
+  }
+  return box(lo[0], lo[1], lo[2], n[0], n[1], n[2], nq);
+}
+
 // The stage in tuned mode: only the faces the stage reads, FAST flux math,
 // tuned register caps.  Returns the number of kernels launched, or -1 when
 // a scratch reset could not be enqueued.
@@ -686,16 +705,9 @@ int stage_tuned(grb_handle* h, const Geo& G, const grb_grid* g, double dt, doubl
   const int gz = G.g, T = 128;
   int launches = 0;
   const double* bf[3] = {old->bx, old->by, old->bz};
-  const int nn[3] = {G.nx, G.ny, G.nz};
   for (int dir = 0; dir < 3; ++dir) {
     KScope ks(h, s, GRB_KIND_FLUX);
-    int lo[3], n[3];
-    for (int a = 0; a < 3; ++a) {
-      if (a == dir) { lo[a] = gz - 1; n[a] = nn[a] + 3; }
-      else if (P.emf == GRB_EMF_GS) { lo[a] = gz - 1; n[a] = nn[a] + 2; }
-      else { lo[a] = gz - 3; n[a] = nn[a] + 6; }  // UCT reconstructs face data across
-    }
-    const Box b = box(lo[0], lo[1], lo[2], n[0], n[1], n[2], G.nq);
+    const Box b = face_box(G, P.emf, dir, G.nq);
     const unsigned nb = nblk(b.count(), T);
     if (dir == 0) launch_flux_tuned<0>(h->var_flux, nb, s, P, G, b, old->state, aux, bf[0], B, h->d_queue + 2);
     if (dir == 1) launch_flux_tuned<1>(h->var_flux, nb, s, P, G, b, old->state, aux, bf[1], B, h->d_queue + 2);
@@ -959,17 +971,13 @@ int grb_advance_substep(grb_handle* h, const grb_grid* g, double t, double dt, d
     CK(cudaGetLastError());
     return GRB_OK;
   }
-  // compute_fluxes: reference ranges (evolve.cpp:908-922)
   const double* bf[3] = {old->bx, old->by, old->bz};
   for (int dir = 0; dir < 3; ++dir) {
-    int lo[3] = {0, 0, 0}, n[3] = {G.NX, G.NY, G.NZ};
-    lo[dir] = gz - 1;
-    n[dir] = (dir == 0 ? G.nx : dir == 1 ? G.ny : G.nz) + 3;
-    const Box b = box(lo[0], lo[1], lo[2], n[0], n[1], n[2], G.nq);
+    const Box b = face_box(G, P.emf, dir, G.nq);
     KScope ks(h, s, GRB_KIND_FLUX);
-    if (dir == 0) k_flux<0><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, old->state, aux, bf[0], B);
-    if (dir == 1) k_flux<1><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, old->state, aux, bf[1], B);
-    if (dir == 2) k_flux<2><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, old->state, aux, bf[2], B);
+    if (dir == 0) k_flux<0, false, kPlainMinB><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, old->state, aux, bf[0], B);
+    if (dir == 1) k_flux<1, false, kPlainMinB><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, old->state, aux, bf[1], B);
+    if (dir == 2) k_flux<2, false, kPlainMinB><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, old->state, aux, bf[2], B);
     ++h->launches;
   }
   const Box eb = box(gz, gz, gz, G.nx + 1, G.ny + 1, G.nz + 1, G.nq);
@@ -989,7 +997,7 @@ int grb_advance_substep(grb_handle* h, const grb_grid* g, double t, double dt, d
     const Box fb = box(gz - 1, gz - 1, gz - 1, G.nx + 2, G.ny + 2, G.nz + 2, G.nq);
     {
     KScope ks(h, s, GRB_KIND_FOFC_FLAG);
-    k_fofc_flag<1><<<nblk(fb.count(), T), T, 0, s>>>(P, G, fb, dt, dtfact, nw->state, old->state, old->bx,
+    k_fofc_flag<kPlainMinB><<<nblk(fb.count(), T), T, 0, s>>>(P, G, fb, dt, dtfact, nw->state, old->state, old->bx,
                                                    old->by, old->bz, g->idx, g->coords, B); ++h->launches;
     }
     {
@@ -1005,7 +1013,7 @@ int grb_advance_substep(grb_handle* h, const grb_grid* g, double t, double dt, d
   const Box ub = box(gz, gz, gz, G.nx, G.ny, G.nz, G.nq);
   {
   KScope ks(h, s, GRB_KIND_UPDATE);
-  k_update<1><<<nblk(ub.count(), T), T, 0, s>>>(P, G, ub, dt, dtfact, nw->state, old->state, aux, g->idx, B); ++h->launches;
+  k_update<kPlainMinB><<<nblk(ub.count(), T), T, 0, s>>>(P, G, ub, dt, dtfact, nw->state, old->state, aux, g->idx, B); ++h->launches;
   }
   if (h->reflux) {
     KScope ks(h, s, GRB_KIND_OTHER);
@@ -1100,10 +1108,10 @@ int grb_compute_auxiliary_quantities_dt(grb_handle* h, const grb_grid* g, const 
     launch_aux_tuned(h->var_aux, nblk(tb.count(), 128), s, h->dp, G, tb, st->state, st->bx, st->by, st->bz, aux,
                      g->idx, g->coords, B, dt_out ? &dta : nullptr, h->d_queue);
   } else if (dt_out) {
-    k_aux<1, true><<<nblk(b.count(), 128), 128, 0, s>>>(h->dp, G, b, st->state, st->bx, st->by, st->bz, aux,
+    k_aux<kPlainMinB, true><<<nblk(b.count(), 128), 128, 0, s>>>(h->dp, G, b, st->state, st->bx, st->by, st->bz, aux,
                                                         g->idx, g->coords, B, dta);
   } else {
-    k_aux<1><<<nblk(b.count(), 128), 128, 0, s>>>(h->dp, G, b, st->state, st->bx, st->by, st->bz, aux, g->idx,
+    k_aux<kPlainMinB><<<nblk(b.count(), 128), 128, 0, s>>>(h->dp, G, b, st->state, st->bx, st->by, st->bz, aux, g->idx,
                                                   g->coords, B);
   }
   ++h->launches;
@@ -2187,10 +2195,7 @@ int grb_autotune(grb_handle* h, const grb_grid* g, const grb_fields* nw, const g
     return best;
   };
   const int gz = G.g;
-  // face fluxes along x with the tuned range
-  int lo[3] = {gz - 1, gz - 1, gz - 1}, n[3] = {G.nx + 3, G.ny + 2, G.nz + 2};
-  if (P.emf == GRB_EMF_UCT) { lo[1] = lo[2] = gz - 3; n[1] = G.ny + 6; n[2] = G.nz + 6; }
-  const Box fbx = box(lo[0], lo[1], lo[2], n[0], n[1], n[2], nt);
+  const Box fbx = face_box(G, P.emf, 0, nt);
   const Box fb = box(gz - 1, gz - 1, gz - 1, G.nx + 2, G.ny + 2, G.nz + 2, nt);
   const Box ub = box(gz, gz, gz, G.nx, G.ny, G.nz, nt);
   Box ab = trimmed(h) ? tuned_aux_box(h, G, s) : box(0, 0, 0, G.NX, G.NY, G.NZ, nt);
@@ -2515,13 +2520,10 @@ extern "C" int grb_advance_substep_static(const grb_params* p, const grb_grid* g
     }
     const double* bf[3] = {obx, oby, obz};
     for (int dir = 0; dir < 3; ++dir) {
-      int lo[3] = {0, 0, 0}, n[3] = {G.NX, G.NY, G.NZ};
-      lo[dir] = gz - 1;
-      n[dir] = (dir == 0 ? G.nx : dir == 1 ? G.ny : G.nz) + 3;
-      const Box b = box(lo[0], lo[1], lo[2], n[0], n[1], n[2], nq);
-      if (dir == 0) k_flux<0><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, os, ax, bf[0], B);
-      if (dir == 1) k_flux<1><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, os, ax, bf[1], B);
-      if (dir == 2) k_flux<2><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, os, ax, bf[2], B);
+      const Box b = face_box(G, P.emf, dir, nq);
+      if (dir == 0) k_flux<0, false, kPlainMinB><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, os, ax, bf[0], B);
+      if (dir == 1) k_flux<1, false, kPlainMinB><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, os, ax, bf[1], B);
+      if (dir == 2) k_flux<2, false, kPlainMinB><<<nblk(b.count(), T), T, 0, s>>>(P, G, b, os, ax, bf[2], B);
     }
     const Box eb = box(gz, gz, gz, G.nx + 1, G.ny + 1, G.nz + 1, nq);
     if (P.emf == GRB_EMF_GS)
@@ -2532,12 +2534,12 @@ extern "C" int grb_advance_substep_static(const grb_params* p, const grb_grid* g
       if (cudaMemsetAsync(B.ftag, 0, L.ftag * nq, s) != cudaSuccess) return GRB_ERR_CUDA;
       if (cudaMemsetAsync(B.etag, 0, L.etag * nq, s) != cudaSuccess) return GRB_ERR_CUDA;
       const Box fb = box(gz - 1, gz - 1, gz - 1, G.nx + 2, G.ny + 2, G.nz + 2, nq);
-      k_fofc_flag<1><<<nblk(fb.count(), T), T, 0, s>>>(P, G, fb, dt, dtfact, ns, os, obx, oby, obz, idx, crd, B);
+      k_fofc_flag<kPlainMinB><<<nblk(fb.count(), T), T, 0, s>>>(P, G, fb, dt, dtfact, ns, os, obx, oby, obz, idx, crd, B);
       k_fofc_faces<false><<<nblk(fb.count(), T), T, 0, s>>>(P, G, fb, os, ax, obx, oby, obz, B);
       k_fofc_edges<<<nblk(fb.count(), T), T, 0, s>>>(G, fb, B);
     }
     const Box ub = box(gz, gz, gz, G.nx, G.ny, G.nz, nq);
-    k_update<1><<<nblk(ub.count(), T), T, 0, s>>>(P, G, ub, dt, dtfact, ns, os, ax, idx, B);
+    k_update<kPlainMinB><<<nblk(ub.count(), T), T, 0, s>>>(P, G, ub, dt, dtfact, ns, os, ax, idx, B);
     k_ct<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, dt, dtfact, nbx, nby, nbz, idx, B);
     if (cudaGetLastError() != cudaSuccess) return GRB_ERR_CUDA;
   }

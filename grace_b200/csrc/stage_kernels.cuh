@@ -1,5 +1,6 @@
 // Per-item kernels of the Cowling GRMHD stage (one thread per face, edge or
-// cell).  Launch ranges and evaluation order follow the reference drivers:
+// cell).  Evaluation order, and launch ranges except the faces' (face_box),
+// follow the reference drivers:
 //   compute_fluxes          src/evolution/evolve.cpp:813-1068, grmhd.hh:551-970
 //   compute_emfs (GS / UCT) src/evolution/evolve.cpp:1069-1340, grmhd_helpers.hh:492-627
 //   flag / apply FOFC       src/evolution/evolve.cpp:456-811

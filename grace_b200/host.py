@@ -467,8 +467,8 @@ class GRMHDEquationsSystem:
         return g[:-1], float(g[-1])
 
     def set_mode(self, mode):
-        """abi.MODE_PLAIN (reference launch ranges, one thread per item) or
-        abi.MODE_TUNED (needed faces only, faster math, tuned variants)."""
+        """abi.MODE_PLAIN (the reference's operations, one thread per item) or
+        abi.MODE_TUNED (staged tiles, faster math, tuned variants)."""
         _lib.check(self.lib.grb_set_mode(self.h, mode), "grb_set_mode")
 
     def autotune(self, new_state, old_state, aux, stream=None):

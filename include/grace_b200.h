@@ -401,12 +401,14 @@ int grb_mlp_grad(grb_handle* h, int64_t n, const float* params,
 
 
 /* ---- execution mode and autotuning --------------------------------------- */
-/* GRB_MODE_PLAIN: one thread per face / edge / cell over the reference's own
- * launch ranges (compute_fluxes computes faces over the full transverse
- * ghost range, evolve.cpp:908-922; linop_apply combines all 23 variables).
- * GRB_MODE_TUNED: only the faces the stage reads (internal scratch), one
- * reciprocal per face for the HLL fluxes, division-free WENO-Z weights, the
- * register-cap variant picked by grb_autotune, fewer divisions in the c2p.
+/* GRB_MODE_PLAIN: one thread per face / edge / cell with the reference's own
+ * operations, on the faces the stage reads (internal scratch; the reference
+ * also computes those of the full transverse ghost range,
+ * evolve.cpp:908-922, which nothing reads); linop_apply combines all 23
+ * variables.
+ * GRB_MODE_TUNED: the same faces from shared-memory tiles, one reciprocal per
+ * face for the HLL fluxes and per WENO-Z state, the register-cap variant
+ * picked by grb_autotune, fewer divisions and evaluations in the c2p.
  * Results agree with the plain mode to rounding.  Which cells the aux pass
  * and linop_apply write is chosen separately, by params.ranges
  * (grb_ranges_kind). */
