@@ -55,6 +55,8 @@ struct grb_handle {
   // learned c2p bracket: FP32 parameter block on the device
   float* d_mlp = nullptr;
   MlpSmem* d_mlp_pack = nullptr;  // shared-memory image of the network
+  float* d_mlp_part = nullptr;    // partial gradients of grb_mlp_grad
+  int mlp_parts = 0;              // rows it holds
   unsigned long long* d_queue = nullptr;  // work-queue counters: [0] aux pass, [1] FOFC flag, [2] flux, [3] update
   double* d_metder = nullptr;             // static-metric cache (grb_set_static_metric)
   size_t metder_bytes = 0;
@@ -870,6 +872,7 @@ int grb_destroy(grb_handle* h) {
   cudaFree(h->d_counters);
   cudaFree(h->d_mlp);
   cudaFree(h->d_mlp_pack);
+  cudaFree(h->d_mlp_part);
   cudaFree(h->d_queue);
   cudaFree(h->d_auxlist);
   cudaFree(h->d_ghostruns);
@@ -1361,6 +1364,7 @@ int grb_mlp_eval(grb_handle* h, int64_t n, const float* params, const float* fea
 }  // extern "C"
 
 namespace {
+constexpr int kKeepParts = 1024;  // 39 MB
 int grad_setup(grb_handle* h) {
   static bool done = false;
   if (!done) {
@@ -1415,15 +1419,31 @@ int grb_mlp_grad(grb_handle* h, int64_t n, const float* params, const float* fea
   if (int rc = grad_setup(h)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   const int nparts = (int)nblk(n, kGradRows);
-  DevBuf part;
-  CK(cudaMalloc(&part.p, sizeof(float) * (size_t)nparts * kPW));
+  // the partial gradients: kept by the handle up to kKeepParts rows (an
+  // allocation and its release took ten times the kernels' time at 16384
+  // samples), larger batches allocate theirs for the call
+  DevBuf own;
+  float* part = nullptr;
+  if (nparts > kKeepParts) {
+    CK(cudaMalloc(&own.p, sizeof(float) * (size_t)nparts * kPW));
+    part = own.as<float>();
+  } else {
+    if (nparts > h->mlp_parts) {
+      cudaFree(h->d_mlp_part);
+      h->d_mlp_part = nullptr;
+      h->mlp_parts = 0;
+      CK(cudaMalloc(&h->d_mlp_part, sizeof(float) * (size_t)nparts * kPW));
+      h->mlp_parts = nparts;
+    }
+    part = h->d_mlp_part;
+  }
   KScope ks(h, s, GRB_KIND_OTHER);
   k_mlp_grad<<<nparts, kGradThreads, sizeof(MlpGradSmem), s>>>(params, n, feat, target, n, 0, 0, 1,
-                                                              1.f / (float)n, part.as<float>());
-  k_mlp_reduce<<<nblk(kPW, 256), 256, 0, s>>>(part.as<float>(), nparts, grad);
+                                                              1.f / (float)n, part);
+  k_mlp_reduce<<<nblk(kPW, kRedCols), 256, 0, s>>>(part, nparts, grad);
   h->launches += 2;
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(s));  // part is freed on return
+  CK(cudaStreamSynchronize(s));  // documented; an own buffer is freed on return
   return GRB_OK;
 }
 
@@ -1514,7 +1534,7 @@ int grb_c2p_train(grb_handle* h, int64_t n, const double* cons, const double* me
     k_mlp_grad<<<nparts, kGradThreads, sizeof(MlpGradSmem), s>>>(h->d_mlp, n, feat.as<float>(), tgt.as<float>(),
                                                                 C.batch, C.seed, it, 0, 1.f / (float)C.batch,
                                                                 part.as<float>());
-    k_mlp_adam<<<nblk(kPW, 256), 256, 0, s>>>(h->d_mlp, m1.as<float>(), m2.as<float>(), part.as<float>(), nparts,
+    k_mlp_adam<<<nblk(kPW, kRedCols), 256, 0, s>>>(h->d_mlp, m1.as<float>(), m2.as<float>(), part.as<float>(), nparts,
                                                (float)lr, (float)(1.0 - b1t), (float)(1.0 - b2t), loss.as<float>(), it);
     h->launches += 2;
   }

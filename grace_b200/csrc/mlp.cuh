@@ -24,6 +24,7 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include <cstddef>
 #include <cstdint>
 
 #include "c2p.cuh"
@@ -600,69 +601,89 @@ __global__ void __launch_bounds__(256) k_mlp_stats(int64_t n, const float* __res
 // y and t normalised.
 constexpr int kGradRows = 64;            // states per CTA
 constexpr int kGradThreads = 256;
-constexpr int kSP = kGradRows + 1;       // pitch of the [feature][state] arrays
+// pitch of the [feature][state] arrays: rows start on 16 bytes and eight
+// consecutive rows on different banks, for 16-byte loads of four states
+constexpr int kSP = kGradRows + 4;
 constexpr int kPW = kMlpNumWeights + 1;  // partial row: gradient, then loss
 
+// 100 KB: two CTAs per SM.  The third layer's activations are last read when
+// its deltas are formed, and leave their place (DB) to the second layer's.
 struct MlpGradSmem {
   MlpSmem net;
   __nv_bfloat16 xs[kGradRows * kXP];
-  float X[kMlpK0 * kSP];
-  float H[3 * kMlpH * kSP];
-  float DA[kMlpH * kSP], DB[kMlpH * kSP];
+  alignas(16) float X[kMlpK0 * kSP];
+  alignas(16) float H[2 * kMlpH * kSP];
+  alignas(16) float DB[kMlpH * kSP];
+  alignas(16) float DA[kMlpH * kSP];
   float y[kGradRows], g[kGradRows], l[kGradRows];
 };
+static_assert(offsetof(MlpGradSmem, DB) == offsetof(MlpGradSmem, H) + sizeof(float) * 2 * kMlpH * kSP,
+              "the third layer's activations continue H");
 
-// dW[o][i] = sum_s D[o][s] Hp[i][s], db[o] = sum_s D[o][s]; thread -> (o, 16 i)
-__device__ __forceinline__ void mlp_wgrad64(const float* D, const float* Hp, float* gW, float* gb) {
-  const int o = threadIdx.x >> 2, q = threadIdx.x & 3;
-  float acc[16], db = 0.f;
+// dW[o][i] = sum_s D[o][s] Hp[i][s], db[o] = sum_s D[o][s], s in order.  A
+// thread takes a 4 x kJ tile (rows o0 + 16 a, columns i0 + 16 b), four states
+// per 16-byte load: (4 + kJ) loads for 16 kJ multiply-adds.
+template <int kJ>
+__device__ __forceinline__ void mlp_wgrad(const float* D, const float* Hp, int ld, float* gW, float* gb) {
+  const int o0 = threadIdx.x >> 4, i0 = threadIdx.x & 15;
+  float acc[4][kJ], db[4];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-  for (int s = 0; s < kGradRows; ++s) {
-    const float d = D[o * kSP + s];
-    db += d;
+  for (int a = 0; a < 4; ++a) {
+    db[a] = 0.f;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j] = fmaf(d, Hp[(q + 4 * j) * kSP + s], acc[j]);
+    for (int j = 0; j < kJ; ++j) acc[a][j] = 0.f;
   }
+#pragma unroll 2
+  for (int s = 0; s < kGradRows; s += 4) {
+    float4 d[4], h[kJ];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) gW[o * kMlpH + q + 4 * j] = acc[j];
-  if (q == 0) gb[o] = db;
-}
-__device__ __forceinline__ void mlp_wgrad16(const float* D, const float* X, float* gW, float* gb) {
-  const int o = threadIdx.x >> 2, q = threadIdx.x & 3;
-  float acc[4], db = 0.f;
+    for (int a = 0; a < 4; ++a) d[a] = *reinterpret_cast<const float4*>(D + (o0 + 16 * a) * kSP + s);
 #pragma unroll
-  for (int j = 0; j < 4; ++j) acc[j] = 0.f;
-  for (int s = 0; s < kGradRows; ++s) {
-    const float d = D[o * kSP + s];
-    db += d;
+    for (int j = 0; j < kJ; ++j) h[j] = *reinterpret_cast<const float4*>(Hp + (i0 + 16 * j) * kSP + s);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = fmaf(d, X[(q + 4 * j) * kSP + s], acc[j]);
-  }
+    for (int a = 0; a < 4; ++a) {
+      db[a] = (((db[a] + d[a].x) + d[a].y) + d[a].z) + d[a].w;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) gW[o * kMlpK0 + q + 4 * j] = acc[j];
-  if (q == 0) gb[o] = db;
-}
-// Dout[i][s] = [Hp[i][s] > 0] sum_o W[o][i] D[o][s]; thread -> (s, 16 i)
-__device__ __forceinline__ void mlp_backdelta(const __nv_bfloat16* W, const float* D, const float* Hp, float* Dout) {
-  const int s = threadIdx.x & (kGradRows - 1), i0 = (threadIdx.x >> 6) * 16;
-  float acc[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-  for (int o = 0; o < kMlpH; ++o) {
-    const float d = D[o * kSP + s];
-    const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(W + o * kPH + i0);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float2 w = __bfloat1622float2(w2[j]);
-      acc[2 * j] = fmaf(w.x, d, acc[2 * j]);
-      acc[2 * j + 1] = fmaf(w.y, d, acc[2 * j + 1]);
+      for (int j = 0; j < kJ; ++j)
+        acc[a][j] = fmaf(d[a].w, h[j].w, fmaf(d[a].z, h[j].z, fmaf(d[a].y, h[j].y, fmaf(d[a].x, h[j].x, acc[a][j]))));
     }
   }
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int i = i0 + j;
-    Dout[i * kSP + s] = Hp[i * kSP + s] > 0.f ? acc[j] : 0.f;
+  for (int a = 0; a < 4; ++a) {
+#pragma unroll
+    for (int j = 0; j < kJ; ++j) gW[(o0 + 16 * a) * ld + i0 + 16 * j] = acc[a][j];
+    if (i0 == 0) gb[o0 + 16 * a] = db[a];
+  }
+}
+// Dout[i][s] = [Hp[i][s] > 0] sum_o W[o][i] D[o][s], o in order; thread -> 4
+// states x 4 inputs.
+__device__ __forceinline__ void mlp_backdelta(const __nv_bfloat16* W, const float* D, const float* Hp, float* Dout) {
+  const int s0 = 4 * (threadIdx.x & 15), i0 = 4 * (threadIdx.x >> 4);
+  float acc[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int s = 0; s < 4; ++s) acc[j][s] = 0.f;
+#pragma unroll 4
+  for (int o = 0; o < kMlpH; ++o) {
+    const float4 d = *reinterpret_cast<const float4*>(D + o * kSP + s0);
+    const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(W + o * kPH + i0);
+    const float2 wa = __bfloat1622float2(w2[0]), wb = __bfloat1622float2(w2[1]);
+    const float w[4] = {wa.x, wa.y, wb.x, wb.y};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[j][0] = fmaf(w[j], d.x, acc[j][0]);
+      acc[j][1] = fmaf(w[j], d.y, acc[j][1]);
+      acc[j][2] = fmaf(w[j], d.z, acc[j][2]);
+      acc[j][3] = fmaf(w[j], d.w, acc[j][3]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 h = *reinterpret_cast<const float4*>(Hp + (i0 + j) * kSP + s0);
+    *reinterpret_cast<float4*>(Dout + (i0 + j) * kSP + s0) =
+        make_float4(h.x > 0.f ? acc[j][0] : 0.f, h.y > 0.f ? acc[j][1] : 0.f, h.z > 0.f ? acc[j][2] : 0.f,
+                    h.w > 0.f ? acc[j][3] : 0.f);
   }
 }
 
@@ -741,23 +762,42 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(const float* __restri
     pg[kMlpNumWeights] = a;
   }
   __syncthreads();
-  mlp_wgrad64(S.DA, H2, pg + kMlpOffW3, pg + kMlpOffB3);
+  mlp_wgrad<4>(S.DA, H2, kMlpH, pg + kMlpOffW3, pg + kMlpOffB3);
   mlp_backdelta(S.net.W3, S.DA, H2, S.DB);
   __syncthreads();
-  mlp_wgrad64(S.DB, H1, pg + kMlpOffW2, pg + kMlpOffB2);
+  mlp_wgrad<4>(S.DB, H1, kMlpH, pg + kMlpOffW2, pg + kMlpOffB2);
   mlp_backdelta(S.net.W2, S.DB, H1, S.DA);
   __syncthreads();
-  mlp_wgrad16(S.DA, S.X, pg + kMlpOffW1, pg + kMlpOffB1);
+  mlp_wgrad<1>(S.DA, S.X, kMlpK0, pg + kMlpOffW1, pg + kMlpOffB1);
 }
 
-// Sum of the partial rows in CTA order -> grad[kPW] (gradient, then loss).
+// Sums over the partial rows of kRedCols parameters (columns) by one CTA of 256
+// threads: kRedSplit threads a column, each a fixed set of rows in order, their
+// sums added in order, so the result does not depend on the run.  Returns
+// column `p`'s sum in the threads of the first kRedCols (p set in those).
+constexpr int kRedCols = 32, kRedSplit = 256 / kRedCols;
+__device__ __forceinline__ bool mlp_column_sum(const float* __restrict__ part, int nparts, int& p, float& g) {
+  __shared__ float red[kRedSplit][kRedCols];
+  const int col = threadIdx.x & (kRedCols - 1), r = threadIdx.x / kRedCols;
+  p = blockIdx.x * kRedCols + col;
+  float a = 0.f;
+  if (p < kPW)
+#pragma unroll 8
+    for (int c = r; c < nparts; c += kRedSplit) a += part[(int64_t)c * kPW + p];
+  red[r][col] = a;
+  __syncthreads();
+  if (r != 0 || p >= kPW) return false;
+  g = red[0][col];
+#pragma unroll
+  for (int k = 1; k < kRedSplit; ++k) g += red[k][col];
+  return true;
+}
+// -> grad[kPW] (gradient, then loss).
 __global__ void __launch_bounds__(256) k_mlp_reduce(const float* __restrict__ part, int nparts,
                                                     float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kPW) return;
-  float g = 0.f;
-  for (int c = 0; c < nparts; ++c) g += part[(int64_t)c * kPW + p];
-  grad[p] = g;
+  int p;
+  float g;
+  if (mlp_column_sum(part, nparts, p, g)) grad[p] = g;
 }
 
 // Adam (Kingma & Ba 2015) on the trainable block; the loss of the step goes
@@ -766,10 +806,9 @@ __global__ void __launch_bounds__(256) k_mlp_adam(float* __restrict__ P, float* 
                                                   float* __restrict__ m2, const float* __restrict__ part,
                                                   int nparts, float lr, float bc1, float bc2,
                                                   float* __restrict__ loss_hist, int64_t step) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kPW) return;
-  float g = 0.f;
-  for (int c = 0; c < nparts; ++c) g += part[(int64_t)c * kPW + p];
+  int p;
+  float g;
+  if (!mlp_column_sum(part, nparts, p, g)) return;
   if (p == kMlpNumWeights) {
     if (loss_hist) loss_hist[step] = g;
     return;
