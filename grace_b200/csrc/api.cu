@@ -243,6 +243,21 @@ PFN_cuTensorMapEncodeTiled_v12000 tma_encoder() {
   }
   return fn;
 }
+// The faces of direction dir that a stage reads: [g-1, n+g+2) along it;
+// across, one row of cells beyond the interior for the Gardiner-Stone edges
+// and the FOFC cells, three for the UCT reconstructions.  The reference
+// computes the whole transverse ghost range (evolve.cpp:908-922): for 16^3
+// blocks 1.8 times as many faces, whose values nothing reads.
+Box face_box(const Geo& G, int emf, int dir, int64_t nq) {
+  const int nn[3] = {G.nx, G.ny, G.nz}, w = emf == GRB_EMF_GS ? 1 : 3;
+  int lo[3], n[3];
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = G.g - (a == dir ? 1 : w);
+    n[a] = nn[a] + (a == dir ? 3 : 2 * w);
+  }
+  return box(lo[0], lo[1], lo[2], n[0], n[1], n[2], nq);
+}
+
 // Tile of direction dir for the face box b (one block's face ranges), for
 // CTAs of nt threads.
 FluxTile flux_tile(int dir, const Geo& G, const Box& b, int nt) {
@@ -295,6 +310,46 @@ bool launch_flux_tma(cudaStream_t s, const DevParams& P, const Geo& G, const Box
   const int nother = dir == 2 ? T.n[1] : T.n[2];
   const dim3 grid((unsigned)((nrow + T.R - 1) / T.R), (unsigned)nother, (unsigned)b.nq);
   k_flux_tma<dir, MINB, NT><<<grid, NT, smem, s>>>(P, G, T, ta, tm, bf, B);
+  return true;
+}
+
+// The three directions in one launch, for grids of at most one wave of CTAs
+// (RK3 step of 8 blocks of 8^3: 232 us against 269 in three launches); false
+// otherwise or when a tile does not fit.  On larger grids the three
+// directions' code, resident together, no longer fits the instruction cache:
+// 64 blocks of 16^3 take 1500 us against 1358.
+constexpr int64_t kFluxMergeTiles = 148 * 4;
+template <int MINB, int NT>
+bool launch_flux_tma3(cudaStream_t s, const DevParams& P, const Geo& G, const double* st, const double* aux,
+                      const double* const bf[3], const StageBufs& B) {
+  FluxTma3 A;
+  size_t smem = 0;
+  int64_t tiles = 0;
+  for (int d = 0; d < 3; ++d) {
+    const Box b = face_box(G, P.emf, d, G.nq);
+    A.T[d] = flux_tile(d, G, b, NT);
+    if (A.T[d].n[0] > NT || b.nq > 65535) return false;
+    if (!make_tmap(&A.aux[d], aux, G, GRB_N_AUX_VARS, b.nq, A.T[d]) ||
+        !make_tmap(&A.met[d], st, G, GRB_N_EVOL_VARS, b.nq, A.T[d]))
+      return false;
+    A.bf[d] = bf[d];
+    smem = std::max(smem, flux_tile_smem(G, A.T[d]));
+    const int nrow = d == 2 ? A.T[d].n[2] : A.T[d].n[1], nother = d == 2 ? A.T[d].n[1] : A.T[d].n[2];
+    A.ntx[d] = (nrow + A.T[d].R - 1) / A.T[d].R;
+    A.first[d] = (int)tiles;
+    tiles += (int64_t)A.ntx[d] * nother;
+  }
+  if (tiles * G.nq > kFluxMergeTiles || tiles > 0x7fffffff) return false;
+  static size_t attr[kMaxDevices] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+  if (smem > attr[dev]) {
+    if (cudaFuncSetAttribute(k_flux_tma3<MINB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+      return false;
+    attr[dev] = smem;
+  }
+  k_flux_tma3<MINB, NT><<<dim3((unsigned)tiles, 1, (unsigned)G.nq), NT, smem, s>>>(P, G, A, B);
   return true;
 }
 
@@ -543,30 +598,42 @@ void launch_aux_tuned(int v, unsigned nb, cudaStream_t s, const DevParams& P, co
 }
 
 // A = b X (+ c Y) on the planes z in [zlo, zlo + nz) and rows y in [ylo,
-// ylo + ny) of a LayoutLeft array (N0, N1, N2, nv_total, nq) at full x
-// extent, for nv variables: each plane's rows are one contiguous span, so
-// every warp reads and writes consecutive doubles.  grid (span / 256,
-// nz * nv, nq); no 64-bit index division.
+// ylo + ny) of LayoutLeft arrays (N0, N1, N2, nv, nq) at full x extent: each
+// plane's rows are one contiguous span, so every warp reads and writes
+// consecutive doubles.  The cell variables and the three face arrays in one
+// launch: grid (spans of 512, planes of the four boxes one after another,
+// nq), two doubles a thread 256 apart; no 64-bit index division.
 struct LinBox {
-  int N0, N1, N2;
+  int N0, N1;
   int ylo, ny, zlo, nz;
   int64_t vstride, qstride;
+  int p0;  // first plane of the box in blockIdx.y
+  double* a;
+  const double* x;
+  const double* y;
 };
-__global__ void __launch_bounds__(256) k_linop_box(LinBox L, int nv, double* __restrict__ a,
-                                                   const double* __restrict__ x, const double* __restrict__ y,
-                                                   double b, double c) {
+struct LinBoxes {
+  LinBox b[4];
+};
+__global__ void __launch_bounds__(256) k_linop_box(LinBoxes S, double b, double c) {
+  const int p = blockIdx.y;
+  const LinBox L = p < S.b[1].p0 ? S.b[0] : p < S.b[2].p0 ? S.b[1] : p < S.b[3].p0 ? S.b[2] : S.b[3];
   const int span = L.ny * L.N0;
-  const int e = blockIdx.x * 256 + threadIdx.x;
+  const int e = blockIdx.x * 512 + threadIdx.x;
   if (e >= span) return;
-  const int zi = blockIdx.y % L.nz, v = blockIdx.y / L.nz;
+  const int v = (p - L.p0) / L.nz, zi = (p - L.p0) - v * L.nz;
   const int64_t o = (int64_t)v * L.vstride + (int64_t)blockIdx.z * L.qstride +
                     ((int64_t)(L.zlo + zi) * L.N1 + L.ylo) * L.N0 + e;
-  a[o] = y ? b * x[o] + c * y[o] : b * x[o];
-}
-void launch_linop_box(cudaStream_t s, const LinBox& L, int nv, int64_t nq, double* a, const double* x,
-                      const double* y, double b, double c) {
-  const dim3 grid((unsigned)((L.ny * L.N0 + 255) / 256), (unsigned)(L.nz * nv), (unsigned)nq);
-  k_linop_box<<<grid, 256, 0, s>>>(L, nv, a, x, y, b, c);
+  const bool two = e + 256 < span;
+  const double x0 = L.x[o], x1 = two ? L.x[o + 256] : 0.0;
+  if (L.y) {
+    const double y0 = L.y[o], y1 = two ? L.y[o + 256] : 0.0;
+    L.a[o] = b * x0 + c * y0;
+    if (two) L.a[o + 256] = b * x1 + c * y1;
+  } else {
+    L.a[o] = b * x0;
+    if (two) L.a[o + 256] = b * x1;
+  }
 }
 
 // The deferred aux pass's cell list: one record per aux cell of the grid, at
@@ -682,32 +749,24 @@ static unsigned fofc_list_grid() {
   return (unsigned)(3 * sms[dev]);
 }
 
-// The faces of direction dir that a stage reads: [g-1, n+g+2) along it;
-// across, one row of cells beyond the interior for the Gardiner-Stone edges
-// and the FOFC cells, three for the UCT reconstructions.  The reference
-// computes the whole transverse ghost range (evolve.cpp:908-922): for 16^3
-// blocks 1.8 times as many faces, whose values nothing reads.
-Box face_box(const Geo& G, int emf, int dir, int64_t nq) {
-  const int nn[3] = {G.nx, G.ny, G.nz}, w = emf == GRB_EMF_GS ? 1 : 3;
-  int lo[3], n[3];
-  for (int a = 0; a < 3; ++a) {
-    lo[a] = G.g - (a == dir ? 1 : w);
-    n[a] = nn[a] + (a == dir ? 3 : 2 * w);
-  }
-  return box(lo[0], lo[1], lo[2], n[0], n[1], n[2], nq);
-}
-
 // The stage in tuned mode: only the faces the stage reads, FAST flux math,
 // tuned register caps.  Returns the number of kernels launched, or -1 when
 // a scratch reset could not be enqueued.
 int stage_tuned(grb_handle* h, const Geo& G, const grb_grid* g, double dt, double dtfact,
                 const grb_fields* nw, const grb_fields* old, const double* aux, cudaStream_t s,
-                StageBufs B, bool count_fofc) {
+                StageBufs B) {
   const DevParams& P = h->dp;
   const int gz = G.g, T = 128;
   int launches = 0;
   const double* bf[3] = {old->bx, old->by, old->bz};
-  for (int dir = 0; dir < 3; ++dir) {
+  bool merged = false;
+  if (h->var_flux == 1 || h->var_flux == 2) {
+    KScope ks(h, s, GRB_KIND_FLUX);
+    merged = h->var_flux == 1 ? launch_flux_tma3<4, 128>(s, P, G, old->state, aux, bf, B)
+                              : launch_flux_tma3<2, 256>(s, P, G, old->state, aux, bf, B);
+    launches += merged;
+  }
+  for (int dir = 0; dir < 3 && !merged; ++dir) {
     KScope ks(h, s, GRB_KIND_FLUX);
     const Box b = face_box(G, P.emf, dir, G.nq);
     const unsigned nb = nblk(b.count(), T);
@@ -719,19 +778,16 @@ int stage_tuned(grb_handle* h, const Geo& G, const grb_grid* g, double dt, doubl
   const Box eb = box(gz, gz, gz, G.nx + 1, G.ny + 1, G.nz + 1, G.nq);
   {
     KScope ks(h, s, GRB_KIND_EMF);
-    if (P.emf == GRB_EMF_GS) k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B);
+    if (P.emf == GRB_EMF_GS) k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B, P.fofc != 0);
     else k_emf_uct<true><<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, old->bx, old->by, old->bz, B);
     ++launches;
   }
   if (P.fofc && P.emf == GRB_EMF_GS) {
     const int64_t nf = G.fcells * G.nq * 3;
-    if (cudaMemsetAsync(B.ftag, 0, (size_t)nf, s) != cudaSuccess ||
-        cudaMemsetAsync(B.etag, 0, (size_t)nf, s) != cudaSuccess ||
-        (count_fofc && cudaMemsetAsync(B.counters, 0, 2 * sizeof(unsigned long long), s) != cudaSuccess))
-      return -1;
+    B.etag = B.ftag + nf;  // this grid's edge tags follow its face tags
+    if (cudaMemsetAsync(B.ftag, 0, (size_t)(2 * nf), s) != cudaSuccess) return -1;
     const Box fb = box(gz - 1, gz - 1, gz - 1, G.nx + 2, G.ny + 2, G.nz + 2, G.nq);
     const bool listed = B.flist && fb.count() < (1ll << 30);
-    if (listed && cudaMemsetAsync(B.fcount, 0, sizeof(uint32_t), s) != cudaSuccess) return -1;
     {
       KScope ks(h, s, GRB_KIND_FOFC_FLAG);
       launch_flag_tuned(h->var_flag, nblk(fb.count(), T), s, P, G, fb, dt, dtfact, nw->state, old->state,
@@ -853,7 +909,7 @@ int grb_create(grb_handle** out, const grb_params* p) {
 
 static void free_scratch(grb_handle* h) {
   cudaFree(h->B.flux); cudaFree(h->B.eface); cudaFree(h->B.vbar); cudaFree(h->B.ecenter);
-  cudaFree(h->B.emf); cudaFree(h->B.ftag); cudaFree(h->B.etag);
+  cudaFree(h->B.emf); cudaFree(h->B.ftag);
   cudaFree(h->B.flist); cudaFree(h->B.fcount);
   h->B.flux = h->B.eface = h->B.vbar = h->B.ecenter = h->B.emf = nullptr;
   h->B.ftag = h->B.etag = nullptr;
@@ -897,7 +953,7 @@ int grb_reserve(grb_handle* h, const grb_grid* g) {
   auto al = [&](void** p, size_t bytes) { return cudaMalloc(p, bytes) == cudaSuccess; };
   bool ok = al((void**)&h->B.flux, sizeof(double) * nf * 7 * 3) &&
             al((void**)&h->B.emf, sizeof(double) * nf * 3) &&
-            al((void**)&h->B.ftag, (size_t)nf * 3) && al((void**)&h->B.etag, (size_t)nf * 3);
+            al((void**)&h->B.ftag, (size_t)nf * 6);  // face tags, then edge tags
   if (ok && h->p.emf == GRB_EMF_GS)
     ok = al((void**)&h->B.eface, sizeof(double) * nf * 2 * 3) &&
          al((void**)&h->B.ecenter, sizeof(double) * nc * 3);
@@ -968,7 +1024,7 @@ int grb_advance_substep(grb_handle* h, const grb_grid* g, double t, double dt, d
   if (h->reflux && (run_offset(h, g) != 0 || g->nq != h->geo.nq)) return fail(h, GRB_ERR_INVALID);
   StageBufs B = run_bufs(h, g);
   if (h->mode == GRB_MODE_TUNED) {
-    const int nl = stage_tuned(h, G, g, dt, dtfact, nw, old, aux, s, B, true);
+    const int nl = stage_tuned(h, G, g, dt, dtfact, nw, old, aux, s, B);
     if (nl < 0) return fail(h, GRB_ERR_CUDA);
     h->launches += nl;
     CK(cudaGetLastError());
@@ -987,16 +1043,15 @@ int grb_advance_substep(grb_handle* h, const grb_grid* g, double t, double dt, d
   {
   KScope ks(h, s, GRB_KIND_EMF);
   if (P.emf == GRB_EMF_GS)
-    k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B);
+    k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B, P.fofc != 0);
   else
     k_emf_uct<false><<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, old->bx, old->by, old->bz, B);
   ++h->launches;
   }
   if (P.fofc && P.emf == GRB_EMF_GS) {
     const int64_t nf = G.fcells * G.nq * 3;
-    CK(cudaMemsetAsync(B.ftag, 0, (size_t)nf, s));
-    CK(cudaMemsetAsync(B.etag, 0, (size_t)nf, s));
-    CK(cudaMemsetAsync(B.counters, 0, 2 * sizeof(unsigned long long), s));
+    B.etag = B.ftag + nf;
+    CK(cudaMemsetAsync(B.ftag, 0, (size_t)(2 * nf), s));
     const Box fb = box(gz - 1, gz - 1, gz - 1, G.nx + 2, G.ny + 2, G.nz + 2, G.nq);
     {
     KScope ks(h, s, GRB_KIND_FOFC_FLAG);
@@ -1172,26 +1227,45 @@ int grb_linop_apply(grb_handle* h, const grb_grid* g, const grb_fields* A, const
     // ghost exchange refills the rest: combine just those.
     const int gz = G.g;
     if (G.nq > 65535 || gz < 2) return fail(h, GRB_ERR_INVALID);
-    LinBox Lc{G.NX, G.NY, G.NZ, gz - 2, G.ny + 4, gz - 2, G.nz + 4, (int64_t)G.cells,
-              (int64_t)G.cells * GRB_N_EVOL_VARS};
-    launch_linop_box(s, Lc, GRB_N_HRSC, G.nq, a[0], x[0], y[0], b, c);
-    ++h->launches;
+    LinBoxes S;
+    S.b[0] = LinBox{G.NX, G.NY, gz - 2, G.ny + 4, gz - 2, G.nz + 4, (int64_t)G.cells,
+                    (int64_t)G.cells * GRB_N_EVOL_VARS, 0, a[0], x[0], y[0]};
+    int planes = GRB_N_HRSC * (G.nz + 4), span = (G.ny + 4) * G.NX;
     for (int fd = 0; fd < 3; ++fd) {
       int N[3] = {G.NX, G.NY, G.NZ}, nn[3] = {G.nx, G.ny, G.nz};
       N[fd] += 1;
       nn[fd] += 1;
       const int64_t fc = (int64_t)N[0] * N[1] * N[2];
-      LinBox Lf{N[0], N[1], N[2], gz, nn[1], gz, nn[2], fc, fc};
-      launch_linop_box(s, Lf, 1, G.nq, a[1 + fd], x[1 + fd], y[1 + fd], b, c);
+      S.b[1 + fd] = LinBox{N[0], N[1], gz, nn[1], gz, nn[2], fc, fc, planes, a[1 + fd], x[1 + fd], y[1 + fd]};
+      planes += nn[2];
+      span = std::max(span, nn[1] * N[0]);
+    }
+    const unsigned spans = (unsigned)((span + 511) / 512);
+    if (planes <= 65535) {
+      k_linop_box<<<dim3(spans, (unsigned)planes, (unsigned)G.nq), 256, 0, s>>>(S, b, c);
       ++h->launches;
+    } else {  // blocks of thousands of planes: one box a launch
+      for (int k = 0; k < 4; ++k) {
+        LinBoxes one = S;
+        one.b[0] = S.b[k];
+        one.b[0].p0 = 0;
+        one.b[1].p0 = one.b[2].p0 = one.b[3].p0 = 1 << 30;
+        const int np = (k == 0 ? GRB_N_HRSC : 1) * S.b[k].nz;
+        k_linop_box<<<dim3(spans, (unsigned)np, (unsigned)G.nq), 256, 0, s>>>(one, b, c);
+        ++h->launches;
+      }
     }
     CK(cudaGetLastError());
     return GRB_OK;
   }
+  LinArrays L;
   for (int v = 0; v < 4; ++v) {
-    k_linop<<<148 * 16, 256, 0, s>>>(n[v], a[v], x[v], y[v], b, c);
-    ++h->launches;
+    L.a[v] = a[v]; L.x[v] = x[v]; L.y[v] = y[v]; L.n[v] = n[v];
+    L.wide[v] = (((uintptr_t)a[v] | (uintptr_t)x[v] | (uintptr_t)y[v]) & 15) == 0;
   }
+  const unsigned lb = (unsigned)std::min<int64_t>(148 * 8, nblk(n[0], 256 * 4));
+  k_linop<<<dim3(lb, 4), 256, 0, s>>>(L, b, c);
+  ++h->launches;
   CK(cudaGetLastError());
   return GRB_OK;
 }
@@ -1734,12 +1808,10 @@ int grb_fill_ghosts_brick_range(grb_handle* h, const grb_grid* g, const grb_fiel
     const int* o = h->ghost_off;
     const int* c = h->ghost_cnt;
     const int mx = std::max({c[0], c[1], c[2]});
-    const dim3 gr((unsigned)((mx + 127) / 128), nfill, 3u);
+    const dim3 gr((unsigned)((std::max(mx, G.NY * G.NZ) + 127) / 128), nfill, 4u);
     k_ghost_runs<<<gr, 128, 0, s>>>(G, br, h->d_ghostruns, make_int3(o[0], o[1], o[2]), make_int3(c[0], c[1], c[2]),
-                                    f->state, bf[1], bf[2]);
-    const dim3 gx((unsigned)((G.NY * G.NZ + 127) / 128), nfill, 1u);
-    k_ghost_xfaces<<<gx, 128, 0, s>>>(G, br, make_fastdiv((uint32_t)G.NY), bf[0]);
-    h->launches += 2;
+                                    make_fastdiv((uint32_t)G.NY), f->state, bf[0], bf[1], bf[2]);
+    ++h->launches;
   } else {
     const dim3 grid((unsigned)((total + 255) / 256), nfill, 4u);
     k_ghost<<<grid, 256, 0, s>>>(G, br, D, f->state, bf[0], bf[1], bf[2]);
@@ -2547,7 +2619,7 @@ extern "C" int grb_advance_substep_static(const grb_params* p, const grb_grid* g
     }
     const Box eb = box(gz, gz, gz, G.nx + 1, G.ny + 1, G.nz + 1, nq);
     if (P.emf == GRB_EMF_GS)
-      k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B);
+      k_emf_gs<<<nblk(eb.count(), T), T, 0, s>>>(G, eb, B, false);
     else
       k_emf_uct<false><<<nblk(eb.count(), T), T, 0, s>>>(P, G, eb, obx, oby, obz, B);
     if (P.fofc && P.emf == GRB_EMF_GS) {

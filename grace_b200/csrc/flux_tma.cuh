@@ -144,19 +144,17 @@ __device__ __forceinline__ void flux_tile_face(const DevParams& P, const Geo& G,
 //   dir 0: lanes i (faces), rows j, other k; box rows j (BY = R, BZ = 1)
 //   dir 1: lanes i, rows j (faces), other k; box rows j - 3 .. (BY = R + 5)
 //   dir 2: lanes i, rows k (faces), other j; box rows k - 3 .. (BZ = R + 5)
-template <int dir, int MINB, int NT = 128>
-__global__ void __launch_bounds__(NT, MINB) k_flux_tma(DevParams P, Geo G, FluxTile T,
-                                                      const __grid_constant__ CUtensorMap tm_aux,
-                                                      const __grid_constant__ CUtensorMap tm_met,
-                                                      const double* __restrict__ bface, StageBufs B) {
+template <int dir>
+__device__ __forceinline__ void flux_tma_tile(const DevParams& P, const Geo& G, const FluxTile& T,
+                                              const CUtensorMap* tm_aux, const CUtensorMap* tm_met,
+                                              const double* __restrict__ bface, const StageBufs& B, int tile,
+                                              int other, int64_t q) {
   extern __shared__ __align__(128) unsigned char sm_raw[];
   const int vs = T.BY * T.BZ * G.NX;  // variable stride in the tile
   const int td = flux_tile_doubles(G, T);
   double* sa = reinterpret_cast<double*>(sm_raw);
   double* sm = sa + td;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + td);
-  const int tile = blockIdx.x, other = blockIdx.y;
-  const int64_t q = blockIdx.z;
   // box origin in cells (x always 0)
   int oy, oz;
   if (dir == 0) { oy = T.lo[1] + tile * T.R; oz = T.lo[2] + other; }
@@ -175,8 +173,8 @@ __global__ void __launch_bounds__(NT, MINB) k_flux_tma(DevParams P, Geo G, FluxT
   if (threadIdx.x == 0 && aligned) {
     const uint32_t bytes = (uint32_t)(2 * 10 * vs * sizeof(double));
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(bytes) : "memory");
-    tma_load5(smem_u32(sa), &tm_aux, 0, oy, oz, 0, (int)q, mb);
-    tma_load5(smem_u32(sm), &tm_met, 0, oy, oz, GRB_GXX, (int)q, mb);
+    tma_load5(smem_u32(sa), tm_aux, 0, oy, oz, 0, (int)q, mb);
+    tma_load5(smem_u32(sm), tm_met, 0, oy, oz, GRB_GXX, (int)q, mb);
   }
   if (!aligned) {
     if (threadIdx.x == 0) atomicOr(B.flags, GRB_FLAG_WAIT_TIMEOUT);
@@ -187,6 +185,38 @@ __global__ void __launch_bounds__(NT, MINB) k_flux_tma(DevParams P, Geo G, FluxT
     return;
   }
   flux_tile_face<dir>(P, G, T, sa, sm, vs, oy, oz, q, bface, B);
+}
+template <int dir, int MINB, int NT = 128>
+__global__ void __launch_bounds__(NT, MINB) k_flux_tma(DevParams P, Geo G, FluxTile T,
+                                                      const __grid_constant__ CUtensorMap tm_aux,
+                                                      const __grid_constant__ CUtensorMap tm_met,
+                                                      const double* __restrict__ bface, StageBufs B) {
+  flux_tma_tile<dir>(P, G, T, &tm_aux, &tm_met, bface, B, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// The three directions in one launch: blockIdx.x runs over the tiles of x,
+// then y, then z (first[d] the first of direction d, ntx[d] its tiles along
+// the row axis).  For small grids, where a direction on its own leaves most
+// SMs idle in its first or last wave.
+struct FluxTma3 {
+  FluxTile T[3];
+  int ntx[3], first[3];
+  const double* bf[3];
+  CUtensorMap aux[3], met[3];
+};
+template <int MINB, int NT>
+__global__ void __launch_bounds__(NT, MINB) k_flux_tma3(DevParams P, Geo G, const __grid_constant__ FluxTma3 A,
+                                                       StageBufs B) {
+  const int x = blockIdx.x;
+  if (x < A.first[1]) {
+    flux_tma_tile<0>(P, G, A.T[0], &A.aux[0], &A.met[0], A.bf[0], B, x % A.ntx[0], x / A.ntx[0], blockIdx.z);
+  } else if (x < A.first[2]) {
+    const int t = x - A.first[1];
+    flux_tma_tile<1>(P, G, A.T[1], &A.aux[1], &A.met[1], A.bf[1], B, t % A.ntx[1], t / A.ntx[1], blockIdx.z);
+  } else {
+    const int t = x - A.first[2];
+    flux_tma_tile<2>(P, G, A.T[2], &A.aux[2], &A.met[2], A.bf[2], B, t % A.ntx[2], t / A.ntx[2], blockIdx.z);
+  }
 }
 
 // The same as a persistent launch (tuned candidate): one wave of CTAs, each

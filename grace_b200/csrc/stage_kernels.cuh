@@ -371,9 +371,15 @@ __device__ __forceinline__ double gs_edge(const Geo& G, const StageBufs& B, int 
 
 // edge range of compute_emfs: [g, n+g] per axis, minus the top along the
 // edge's own direction (evolve.cpp:1089-1103)
-__global__ void __launch_bounds__(128) k_emf_gs(Geo G, Box box, StageBufs B) {
+// zero: also clears the stage's FOFC counters, which the kernels after it add
+// to (three 4 to 16 byte memsets less on the stream).
+__global__ void __launch_bounds__(128) k_emf_gs(Geo G, Box box, StageBufs B, bool zero) {
   int i, j, k;
   int64_t q;
+  if (zero && blockIdx.x == 0 && threadIdx.x == 0) {
+    B.counters[0] = B.counters[1] = 0;
+    if (B.fcount) *B.fcount = 0;
+  }
   if (!decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q)) return;
   if (i < G.nx + G.g) B.emf[emi(G, i, j, k, 0, q)] = gs_edge(G, B, 0, i, j, k, q);
   if (j < G.ny + G.g) B.emf[emi(G, i, j, k, 1, q)] = gs_edge(G, B, 1, i, j, k, q);
@@ -1225,11 +1231,50 @@ __global__ void k_reset_diag(Geo G, double* __restrict__ aux) {
   }
 }
 
-// linop_apply: a = b*x (+ c*y) elementwise, 2 doubles per thread
-__global__ void k_linop(int64_t n, double* __restrict__ a, const double* __restrict__ x,
-                        const double* __restrict__ y, double b, double c) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-    a[t] = y ? b * x[t] + c * y[t] : b * x[t];
+// linop_apply: a = b*x (+ c*y) elementwise on the four arrays (blockIdx.y: the
+// cell variables, the x, y, z faces) in one launch: the face arrays are a
+// tenth of the work, and one launch at a time left the GPU half empty on
+// small grids.  Two doubles a load where the array's pointers allow it.
+// a may be x or y.
+struct LinArrays {
+  double* a[4];
+  const double* x[4];
+  const double* y[4];
+  int64_t n[4];
+  bool wide[4];  // 16-byte aligned pointers
+};
+__global__ void __launch_bounds__(256) k_linop(LinArrays L, double b, double c) {
+  // the array's entries by select (a dynamic index into the parameter would
+  // copy it to local memory)
+  const int v = blockIdx.y;
+  double* a = v == 0 ? L.a[0] : v == 1 ? L.a[1] : v == 2 ? L.a[2] : L.a[3];
+  const double* x = v == 0 ? L.x[0] : v == 1 ? L.x[1] : v == 2 ? L.x[2] : L.x[3];
+  const double* y = v == 0 ? L.y[0] : v == 1 ? L.y[1] : v == 2 ? L.y[2] : L.y[3];
+  const int64_t n = v == 0 ? L.n[0] : v == 1 ? L.n[1] : v == 2 ? L.n[2] : L.n[3];
+  const bool wide = v == 0 ? L.wide[0] : v == 1 ? L.wide[1] : v == 2 ? L.wide[2] : L.wide[3];
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  if (!wide) {
+    for (int64_t t = t0; t < n; t += step) a[t] = y ? b * x[t] + c * y[t] : b * x[t];
+    return;
+  }
+  const int64_t h = n / 2;
+  double2* a2 = reinterpret_cast<double2*>(a);
+  const double2* x2 = reinterpret_cast<const double2*>(x);
+  const double2* y2 = reinterpret_cast<const double2*>(y);
+  if (y) {
+#pragma unroll 2
+    for (int64_t t = t0; t < h; t += step) {
+      const double2 u = x2[t], w = y2[t];
+      a2[t] = make_double2(b * u.x + c * w.x, b * u.y + c * w.y);
+    }
+  } else {
+#pragma unroll 2
+    for (int64_t t = t0; t < h; t += step) {
+      const double2 u = x2[t];
+      a2[t] = make_double2(b * u.x, b * u.y);
+    }
+  }
+  if (t0 == 0 && (n & 1)) a[n - 1] = y ? b * x[n - 1] + c * y[n - 1] : b * x[n - 1];
 }
 // the three-term linop_apply: a = b*x + c*y + d*z elementwise, the sums
 // left to right.  a may be any of x, y, z (each element is read before it
@@ -1332,7 +1377,7 @@ __global__ void __launch_bounds__(256) k_ghost(Geo G, Brick br, GhostDivs D, dou
 // throughout.  Each thread loads up to 8 of its row's sources before it
 // stores them, so the copies of a row overlap; the source of every face is
 // the one k_ghost maps it to.
-__global__ void __launch_bounds__(128) k_ghost_xfaces(Geo G, Brick br, FastDiv dny, double* __restrict__ fx) {
+__device__ __forceinline__ void ghost_xfaces(const Geo& G, const Brick& br, const FastDiv& dny, double* __restrict__ fx) {
   const int N0 = G.NX + 1, N1 = G.NY;
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= N1 * G.NZ) return;
@@ -1376,14 +1421,20 @@ __global__ void __launch_bounds__(128) k_ghost_xfaces(Geo G, Brick br, FastDiv d
 // extents along x that are multiples of 4 (so runs never straddle the
 // interior's edge) on arrays whose rows are 4-aligned (not staggered along
 // x): blockIdx.z = 0 the cell-centred HRSC variables, 1, 2 the face arrays
-// staggered along y, z; runs + off[a] lists array a's ghost runs, packed
+// staggered along y, z, 3 the x face array by rows (ghost_xfaces; in the
+// same launch, since neither fills the GPU on its own for long); runs + off[a] lists array a's ghost runs, packed
 // r | j << 8 | k << 16 (x in [4r, 4r + 4) of row (j, k)).  Each thread
 // copies one run with 16-byte loads and stores: the matching run of its
 // source row, or one cell repeated where zero-gradient applies along x.
 __global__ void __launch_bounds__(128) k_ghost_runs(Geo G, Brick br, const uint32_t* __restrict__ runs,
-                                                   int3 off, int3 cnt, double* __restrict__ cells,
-                                                   double* __restrict__ fy, double* __restrict__ fz) {
+                                                   int3 off, int3 cnt, FastDiv dny, double* __restrict__ cells,
+                                                   double* __restrict__ fx, double* __restrict__ fy,
+                                                   double* __restrict__ fz) {
   const int arr = blockIdx.z;
+  if (arr == 3) {
+    ghost_xfaces(G, br, dny, fx);
+    return;
+  }
   const int len = arr == 0 ? cnt.x : arr == 1 ? cnt.y : cnt.z;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= len) return;
