@@ -57,7 +57,8 @@ __device__ __forceinline__ int list_var(const RestrictVars& V, int i) {
 
 // Cell variables.  box: (n/2)^3 coarse cells x (nvars_in_list x nquads)
 // folded into the box's block index (variable fastest).  kHigh: the 5-point
-// Lagrange operator, else the 8-cell average.
+// Lagrange operator (blocks of 4 cells along z too wide for k_restrict_lag),
+// else the 8-cell average.
 template <bool kHigh>
 __global__ void __launch_bounds__(128) k_restrict_cells(Geo G, Box box, RestrictVars V, FastDiv dnv,
                                                         const double* __restrict__ src, double* __restrict__ dst,
@@ -106,7 +107,62 @@ __global__ void __launch_bounds__(128) k_restrict_cells(Geo G, Box box, Restrict
   dst[(dst_q[iq] * GRB_N_EVOL_VARS + v) * G.cells + ((int64_t)(k + G.g) * N1 + (j + G.g)) * N0 + (i + G.g)] = r;
 }
 
-// High-order list, one thread per (i, j) column of coarse cells and
+// High-order list, one CTA per variable of a quadrant: the 5-point Lagrange
+// restriction axis by axis, the x and then the y contractions of the whole
+// interior in shared memory ((nx/2) ny nz + (nx/2) (ny/2) nz doubles: 24 KB
+// for 16^3).  Every fine row is contracted once, where a thread per column of
+// coarse cells (k_restrict_lag_zcol) repeats each x contraction for the up
+// to three columns that share it and was bound by its 25 loads a plane.  512
+// blocks of 16^3, restricted and prolonged (23 variables, face B, three
+// element kinds): 514 us by columns, 429 us with this and k_prolong_lag.  The
+// operands and their order are lagrange_restrict_op<4>'s: x, y, z.
+// dx, dy: divisors nx/2 and ny (pass x), dz: ny/2.
+__global__ void __launch_bounds__(128) k_restrict_lag(Geo G, RestrictVars V, FastDiv dnv, FastDiv dx, FastDiv dy,
+                                                      FastDiv dz, const double* __restrict__ src,
+                                                      double* __restrict__ dst, const int64_t* __restrict__ src_q,
+                                                      const int64_t* __restrict__ dst_q,
+                                                      const uint8_t* __restrict__ child) {
+  extern __shared__ __align__(16) double sm_fmr[];
+  const uint32_t iq = fast_div(blockIdx.x, dnv);
+  const int v = list_var(V, (int)(blockIdx.x - iq * (uint32_t)V.n));
+  const int N0 = G.NX, N1 = G.NY, g = G.g;
+  const int hx = G.nx / 2, hy = G.ny / 2, hz = G.nz / 2;
+  const double* u = src + (src_q[iq] * GRB_N_EVOL_VARS + v) * G.cells;
+  double* o = dst + (dst_q[iq] * GRB_N_EVOL_VARS + v) * G.cells;
+  const uint8_t cid = child[iq];
+  double* X = sm_fmr;                  // [nz][ny][hx]
+  double* Y = X + hx * G.ny * G.nz;    // [nz][hy][hx]
+  for (int t = threadIdx.x; t < hx * G.ny * G.nz; t += 128) {
+    const uint32_t r = fast_div((uint32_t)t, dx), z = fast_div(r, dy);
+    const int i = t - (int)r * hx, y = (int)(r - z * (uint32_t)G.ny);
+    const int fi = 2 * i + g, ox = lag4_offset(fi, G.nx, g, cid & 1);
+    const double* l = u + ((int64_t)((int)z + g) * N1 + (y + g)) * N0 + fi + ox - 3;
+    const double line[5] = {l[0], l[1], l[2], l[3], l[4]};
+    X[t] = contract5_rn(c_restrict5 + 5 * ox, line);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < hx * hy * G.nz; t += 128) {
+    const uint32_t r = fast_div((uint32_t)t, dx), z = fast_div(r, dz);
+    const int i = t - (int)r * hx, j = (int)(r - z * (uint32_t)hy);
+    const int fj = 2 * j + g, oy = lag4_offset(fj, G.ny, g, (cid >> 1) & 1);
+    const double* l = X + ((int)z * G.ny + 2 * j + oy - 3) * hx + i;
+    const double line[5] = {l[0], l[hx], l[2 * hx], l[3 * hx], l[4 * hx]};
+    Y[t] = contract5_rn(c_restrict5 + 5 * oy, line);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < hx * hy * hz; t += 128) {
+    const uint32_t r = fast_div((uint32_t)t, dx), kz = fast_div(r, dz);
+    const int i = t - (int)r * hx, j = (int)(r - kz * (uint32_t)hy), k = (int)kz;
+    const int oz = lag4_offset(2 * k + g, G.nz, g, (cid >> 2) & 1);
+    const int s = hx * hy;
+    const double* l = Y + (2 * k + oz - 3) * s + j * hx + i;
+    const double line[5] = {l[0], l[s], l[2 * s], l[3 * s], l[4 * s]};
+    o[((int64_t)(k + g) * N1 + (j + g)) * N0 + (i + g)] = contract5_rn(c_restrict5 + 5 * oz, line);
+  }
+}
+
+// High-order list of blocks whose contractions do not fit shared memory
+// (interiors above 28^3), one thread per (i, j) column of coarse cells and
 // variable, walking the column along z: each fine plane's contractions along
 // x and y (with the column's x and y stencils) are computed once and the
 // last five kept in registers; coarse cell k takes the z contraction of the
@@ -114,8 +170,8 @@ __global__ void __launch_bounds__(128) k_restrict_cells(Geo G, Box box, Restrict
 // reached the last of them.  Stencil windows never move back along z (the
 // edge and half-dependent offsets keep their ends non-decreasing), so one
 // pass over the fine planes ngz .. nz + ngz - 1 serves every cell.  The
-// operands and their order are those of k_restrict_cells<true>, bit for
-// bit.  box: (nx/2, ny/2, 1) x (nvars_in_list x nquads), variable fastest.
+// operands and their order are those of k_restrict_lag, bit for bit.  512
+// blocks of 16^3, 16 variables: 170 us.  box: (nx/2, ny/2, 1) x (nvars_in_list x nquads), variable fastest.
 __global__ void __launch_bounds__(128) k_restrict_lag_zcol(Geo G, Box box, RestrictVars V, FastDiv dnv,
                                                            const double* __restrict__ src, double* __restrict__ dst,
                                                            const int64_t* __restrict__ src_q,
@@ -283,7 +339,86 @@ __global__ void __launch_bounds__(128) k_prolong_cells(Geo G, Box box, RestrictV
     }
 }
 
-// High-order list, one thread per (x, y) column of an element's coarse
+// High-order list, one CTA per element and kV of the list's variables: the
+// 5-point Lagrange prolongation axis by axis.  With r coarse cells along
+// each axis of the element's region (window r + 4): both x halves of the
+// window's rows, then both y halves, in shared memory, then both z halves
+// stored.  Each contraction is made once and the loads of a CTA's variables
+// are in flight together (a single element's few hundred loads, staged
+// behind one barrier, leave the SM waiting); a thread per column
+// (k_prolong_lag_zcol) repeats the x and y contractions of the rows that
+// neighbouring columns share, 25 loads a plane.  Operands and order are
+// lagrange_prolong_op<4>'s.  D: divisors of the possible extents, 0: n/2,
+// 1: ngz/2, 2: n/2 + 4, 3: ngz/2 + 4, 4: n, 5: ngz.
+struct ProlongDivs {
+  FastDiv d[6];
+};
+template <int kKind, int kV>
+__global__ void __launch_bounds__(256) k_prolong_lag(Geo G, RestrictVars V, FastDiv dgroups, ProlongDivs D,
+                                                     const double* __restrict__ cbuf, double* __restrict__ fine,
+                                                     const int64_t* __restrict__ fine_q,
+                                                     const int64_t* __restrict__ cbuf_q,
+                                                     const uint8_t* __restrict__ elem) {
+  extern __shared__ __align__(16) double sm_fmr[];
+  const uint32_t iq = fast_div(blockIdx.x, dgroups);
+  const int v0 = (int)(blockIdx.x - iq * dgroups.d) * kV;
+  const int nv = min(kV, V.n - v0);
+  const int e = elem[iq], n = G.nx, g = G.g;
+  int r[3], k0[3], f0[3];
+  bool along[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    int w, lp;
+    ghost_axis<kKind>(e, d, w, lp);
+    along[d] = w == 2;
+    r[d] = along[d] ? n / 2 : g / 2;
+    k0[d] = ghost_idx(w, n / 2, g, g / 2, 0);
+    f0[d] = ghost_idx(w, n, g, 0, 0);
+  }
+  const FastDiv drx = along[0] ? D.d[0] : D.d[1], dwy = along[1] ? D.d[2] : D.d[3], dwz = along[2] ? D.d[2] : D.d[3];
+  const FastDiv dfx = along[0] ? D.d[4] : D.d[5], dry = along[1] ? D.d[0] : D.d[1], dfy = along[1] ? D.d[4] : D.d[5];
+  const FastDiv drz = along[2] ? D.d[0] : D.d[1];
+  const int wy = r[1] + 4, wz = r[2] + 4, fx = 2 * r[0], fy = 2 * r[1];
+  const int N0 = G.NX, N1 = G.NY;
+  double* X = sm_fmr;                      // [nv][wz][wy][fx]
+  double* Y = X + (int64_t)kV * wz * wy * fx;  // [nv][wz][fy][fx]
+  const double* ub = cbuf + cbuf_q[iq] * GRB_N_EVOL_VARS * G.cells;
+  double* ob = fine + fine_q[iq] * GRB_N_EVOL_VARS * G.cells;
+  for (int t = threadIdx.x; t < nv * wz * wy * r[0]; t += 256) {
+    const uint32_t a = fast_div((uint32_t)t, drx), b = fast_div(a, dwy), c = fast_div(b, dwz);
+    const int x = t - (int)a * r[0], y = (int)(a - b * (uint32_t)wy), z = (int)(b - c * (uint32_t)wz);
+    const double* l = ub + list_var(V, v0 + (int)c) * G.cells +
+                      ((int64_t)(k0[2] + z - 2) * N1 + (k0[1] + y - 2)) * N0 + k0[0] + x - 2;
+    const double line[5] = {l[0], l[1], l[2], l[3], l[4]};
+    double* s = X + (int)a * fx + 2 * x;
+    s[0] = contract5_rn(c_prolong5, line);
+    s[1] = contract5_rn(c_prolong5 + 5, line);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < nv * wz * r[1] * fx; t += 256) {
+    const uint32_t a = fast_div((uint32_t)t, dfx), b = fast_div(a, dry);  // b = variable x plane
+    const int x = t - (int)a * fx, y = (int)(a - b * (uint32_t)r[1]);
+    const double* l = X + ((int)b * wy + y) * fx + x;
+    const double line[5] = {l[0], l[fx], l[2 * fx], l[3 * fx], l[4 * fx]};
+    double* s = Y + ((int)b * fy + 2 * y) * fx + x;
+    s[0] = contract5_rn(c_prolong5, line);
+    s[fx] = contract5_rn(c_prolong5 + 5, line);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < nv * r[2] * fy * fx; t += 256) {
+    const uint32_t a = fast_div((uint32_t)t, dfx), b = fast_div(a, dfy), c = fast_div(b, drz);
+    const int x = t - (int)a * fx, y = (int)(a - b * (uint32_t)fy), z = (int)(b - c * (uint32_t)r[2]);
+    const int s = fx * fy;
+    const double* l = Y + ((int)c * wz + z) * s + y * fx + x;
+    const double line[5] = {l[0], l[s], l[2 * s], l[3 * s], l[4 * s]};
+    double* o = ob + list_var(V, v0 + (int)c) * G.cells + ((int64_t)(f0[2] + 2 * z) * N1 + (f0[1] + y)) * N0 + f0[0] + x;
+    o[0] = contract5_rn(c_prolong5, line);
+    o[(int64_t)N1 * N0] = contract5_rn(c_prolong5 + 5, line);
+  }
+}
+
+// High-order list of blocks whose contractions do not fit shared memory
+// (k_prolong_lag), one thread per (x, y) column of an element's coarse
 // region and variable, walking the column along z: each z plane's x sums
 // (both x halves) and y sums (the 4 (x, y) halves) are computed once and the
 // last five planes' y sums kept in registers, from which every coarse cell

@@ -1449,6 +1449,26 @@ int grad_setup(grb_handle* h) {
 }
 }  // namespace
 
+// Shared memory a CTA of the FMR kernels may take (two per SM), and the
+// attribute that allows it, per kernel and device.
+constexpr size_t kFmrSmem = 100 << 10;
+template <class... A>
+static bool fmr_smem(void (*kernel)(A...)) {
+  static void* done[kMaxDevices][8] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+  for (void*& k : done[dev]) {
+    if (k == reinterpret_cast<void*>(kernel)) return true;
+    if (!k) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFmrSmem) != cudaSuccess)
+        return false;
+      k = reinterpret_cast<void*>(kernel);
+      return true;
+    }
+  }
+  return false;
+}
+
 // FMR prolongation launches of one element kind (grb_prolong_to_ghosts).
 template <int kKind>
 static void launch_prolong(const Geo& G, const int ext[3], const grb_fields* fine, const grb_fields* cbuf,
@@ -1459,7 +1479,26 @@ static void launch_prolong(const Geo& G, const int ext[3], const grb_fields* fin
     k_prolong_cells<kKind><<<nblk(b.count(), 128), 128, 0, s>>>(G, b, V[0], make_fastdiv((uint32_t)V[0].n),
                                                                 cbuf->state, fine->state, fine_q, cbuf_q, elem_id);
   }
-  if (V[1].n) {
+  // variables per CTA of k_prolong_lag: as many as give its 256 threads a few
+  // items each and let several CTAs share an SM
+  constexpr int kV = kKind == GRB_ELEM_FACE ? 2 : (kKind == GRB_ELEM_EDGE ? 4 : 8);
+  size_t smem = 0;
+  for (int o = 0; o < 3; ++o) {  // the kind's orientations (ghost extent along one, two or three axes)
+    int r[3];
+    for (int d = 0; d < 3; ++d) {
+      const bool along = kKind == GRB_ELEM_FACE ? d != o : (kKind == GRB_ELEM_EDGE ? d == o : false);
+      r[d] = along ? G.nx / 2 : G.g / 2;
+    }
+    smem = std::max(smem, sizeof(double) * kV * 2 * r[0] * (r[2] + 4) * (size_t)(r[1] + 4 + 2 * r[1]));
+  }
+  const int groups = (V[1].n + kV - 1) / kV;
+  if (V[1].n && smem <= kFmrSmem && groups * nelems <= 0x7fffffff && fmr_smem(k_prolong_lag<kKind, kV>)) {
+    ProlongDivs D;
+    const int ext6[6] = {G.nx / 2, G.g / 2, G.nx / 2 + 4, G.g / 2 + 4, G.nx, G.g};
+    for (int k = 0; k < 6; ++k) D.d[k] = make_fastdiv((uint32_t)ext6[k]);
+    k_prolong_lag<kKind, kV><<<(unsigned)(groups * nelems), 256, smem, s>>>(
+        G, V[1], make_fastdiv((uint32_t)groups), D, cbuf->state, fine->state, fine_q, cbuf_q, elem_id);
+  } else if (V[1].n) {
     // the kind's largest element cross-section in (x, y), in coarse cells
     const int ne = kKind == GRB_ELEM_FACE ? 6 : (kKind == GRB_ELEM_EDGE ? 12 : 8);
     int cols = 0;
@@ -2008,18 +2047,28 @@ int grb_restrict_to_coarse(grb_handle* h, const grb_grid* g, const grb_fields* f
     }
     if ((int64_t)nl * nquads >= (1ll << 32)) return fail(h, GRB_ERR_INVALID);
     const Box b = box(0, 0, 0, G.nx / 2, G.ny / 2, G.nz / 2, (int64_t)nl * nquads);
-    if (pass == 0)
+    if (pass == 0) {
       k_restrict_cells<false><<<nblk(b.count(), 128), 128, 0, s>>>(G, b, V, make_fastdiv((uint32_t)nl), fine->state,
                                                                    cbuf->state, src_q, dst_q, child_id);
-    else if (G.nz >= 6) {
-      // by z columns; with 4 cells along z the edge stencils' windows move
-      // back along z, so those blocks keep one thread per coarse cell
-      const Box bc = box(0, 0, 0, G.nx / 2, G.ny / 2, 1, (int64_t)nl * nquads);
-      k_restrict_lag_zcol<<<nblk(bc.count(), 128), 128, 0, s>>>(G, bc, V, make_fastdiv((uint32_t)nl), fine->state,
-                                                               cbuf->state, src_q, dst_q, child_id);
-    } else
-      k_restrict_cells<true><<<nblk(b.count(), 128), 128, 0, s>>>(G, b, V, make_fastdiv((uint32_t)nl), fine->state,
-                                                                  cbuf->state, src_q, dst_q, child_id);
+    } else {
+      const size_t smem = sizeof(double) * ((size_t)G.nx / 2 * G.ny * G.nz + (size_t)G.nx / 2 * (G.ny / 2) * G.nz);
+      // below 6 cells along y or z the stencils reach ghost cells, which the
+      // staged interior does not hold
+      if (G.ny >= 6 && G.nz >= 6 && smem <= kFmrSmem && (int64_t)nl * nquads <= 0x7fffffff &&
+          fmr_smem(k_restrict_lag)) {
+        k_restrict_lag<<<(unsigned)(nl * nquads), 128, smem, s>>>(
+            G, V, make_fastdiv((uint32_t)nl), make_fastdiv((uint32_t)G.nx / 2), make_fastdiv((uint32_t)G.ny),
+            make_fastdiv((uint32_t)G.ny / 2), fine->state, cbuf->state, src_q, dst_q, child_id);
+      } else if (G.nz < 6) {
+        // with 4 cells along z the edge stencils' windows move back along z
+        k_restrict_cells<true><<<nblk(b.count(), 128), 128, 0, s>>>(G, b, V, make_fastdiv((uint32_t)nl), fine->state,
+                                                                    cbuf->state, src_q, dst_q, child_id);
+      } else {
+        const Box bc = box(0, 0, 0, G.nx / 2, G.ny / 2, 1, (int64_t)nl * nquads);
+        k_restrict_lag_zcol<<<nblk(bc.count(), 128), 128, 0, s>>>(G, bc, V, make_fastdiv((uint32_t)nl), fine->state,
+                                                                 cbuf->state, src_q, dst_q, child_id);
+      }
+    }
     ++h->launches;
   }
   const double* fs[3] = {fine->bx, fine->by, fine->bz};
