@@ -559,15 +559,20 @@ __device__ __forceinline__ void fofc_flag_cell(const DevParams& P, const Geo& G,
   if (P.dmp_enable) {
     const int lv[2] = {GRB_DENS, GRB_TAU};
     for (int n = 0; n < 2 && !dmp; ++n) {
+      const double t = c[lv[n]];
+      const double* w = u + G.cells * lv[n];
+      // The window's largest value is at least the cell's own and its least at
+      // most that (and rounding keeps the order), so a value within M of the
+      // cell's own passes: the 27 loads are for the few others.
+      if (P.dmp_M > 0.0 && t <= P.dmp_M * w[0] && t >= w[0] * P.idmp_M) continue;
       double vmax = -1.7976931348623157e308, vmin = 1.7976931348623157e308;
       for (int kt = -1; kt <= 1; ++kt)
         for (int jt = -1; jt <= 1; ++jt)
           for (int it = -1; it <= 1; ++it) {
-            const double v = u[G.cells * lv[n] + it + (int64_t)G.NX * (jt + G.NY * kt)];
+            const double v = w[it + (int64_t)G.NX * (jt + G.NY * kt)];
             vmax = v > vmax ? v : vmax;
             vmin = v < vmin ? v : vmin;
           }
-      const double t = c[lv[n]];
       if (t > P.dmp_M * vmax || t < vmin * P.idmp_M) dmp = true;
     }
   }
