@@ -1305,6 +1305,13 @@ int launch_c2p(grb_handle* h, int64_t n, const double* cons, const double* metri
   if (n > (int64_t)kC2PThreads * 0x7fffffff) return fail(h, GRB_ERR_INVALID);
   const unsigned nb = nblk(n, kC2PThreads);
   const bool fast = h->mode == GRB_MODE_TUNED;
+  if (fast && !learned && n <= kC2PDirect) {
+    k_c2p_batch_front<false, false><<<nb, kC2PThreads, 0, s>>>(h->dp, n, cons, metric, prims, cons_out, err, d,
+                                                              nullptr, h->d_flags, nullptr, nullptr);
+    ++h->launches;
+    CK(cudaGetLastError());
+    return GRB_OK;
+  }
   if (fast) {
     // tuned mode: the entropy backups deferred to a second, compacted pass
     if (n > h->defer_cap) {

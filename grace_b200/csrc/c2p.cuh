@@ -731,6 +731,23 @@ GRB_HD void kscf(const DevEos& e, const Met& m, const double c[10], KScF& k) {
   k.ow = rcp_f(1.0 + zs);
 }
 
+// What a root solve and the primitives from it need of a state: the scalars,
+// r^i and the entropy D s / D.  The conservatives and the metric are dead
+// across the solve (the few states that need the metric again get it from a
+// functor that reloads it), which is what keeps the solve's registers few.
+struct C2PLive {
+  KScF k;
+  double rup[3], s;
+};
+template <bool kRound>
+GRB_HD void c2p_live(const DevEos& e, const Met& m, const double c[10], C2PLive& L) {
+  kscf<kRound>(e, m, c, L.k);
+  mvs(m.gi, c + 1, L.rup);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) L.rup[i] *= L.k.iD;
+  L.s = c[6] * L.k.iD;
+}
+
 // Cold part of the hybrid EOS at rho: P_cold / rho and eps_cold.
 GRB_HD void pw_cold_f(const DevEos& e, double& rho, double irho, double& pr, double& ec) {
   const int i = pw_idx(e, rho);
@@ -991,37 +1008,39 @@ GRB_HD double mu0_f(const DevEos& e, const KScF& k) {
   return mu0;
 }
 
-// Writes the primitives of a solution (Kastaun's or the entropy's) and its
-// W, B.z and b^2.
-template <class Fn>
-GRB_HD void take_solution(const DevEos& e, const Met& m, const KScF& k, const Fn& f, double mu, const double c[10],
-                          double pr[13], WB& wb, bool& wb_ok) {
+// Writes the primitives of a solution (Kastaun's or the entropy's; prims'
+// B set) and its W, B.z and b^2; met(): the state's metric, for the velocity
+// limit, where they come from the primitives.
+template <class Fn, class MetF>
+GRB_HD void take_solution(const DevEos& e, const C2PLive& L, const Fn& f, double mu, double pr[13], WB& wb,
+                          MetF&& met) {
+  const KScF& k = L.k;
   const double rho = clamp_f(f.rho, e.rhomin, e.rhomax);
   pr[GRB_P_RHO] = rho;
   pr[GRB_P_EPS] = f.eps;
   pr[GRB_P_PRESS] = f.prho * rho;
   pr[GRB_P_TEMP] = e.kind == GRB_EOS_IDEAL_GAS ? f.eth * e.gm1 : fmax(0.0, f.eth * e.gthm1);
-  double rup[3];
-  mvs(m.gi, c + 1, rup);
   const double kz = f.w * mu * f.x, kb = mu * k.rBt * k.isD;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) pr[GRB_P_ZX + i] = kz * (rup[i] * k.iD + kb * c[7 + i]);
+  for (int i = 0; i < 3; ++i) pr[GRB_P_ZX + i] = kz * (L.rup[i] + kb * pr[GRB_P_BX + i]);
   wb.W = f.w;
   wb.iW = f.iw;
   wb.z2 = f.w * f.w - 1.0;
   wb.Bz = f.w * mu * (k.rBt * (k.isD * k.D));
   wb.b2 = (k.b2 * k.D + wb.Bz * wb.Bz) * (f.iw * f.iw);
-  wb_ok = !f.vhigh;
+  if (f.vhigh) wb = wb_of(met(), pr);
 }
 
 // c2p_front in the tuned mode (plain bracket).
 // kBrent: the root by Brent's iteration from the plain bracket (the batch
 // entry points), else by secant_root (the stage passes).
-template <bool kBrent, bool kDry = false>
-GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const DevParams& P, double alp_bh_thresh) {
+template <bool kBrent, bool kDry = false, class MetF>
+GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const DevParams& P, double alp_bh_thresh,
+                            C2PLive& L, MetF&& met) {
   C2PState F{};
   const DevEos& e = P.eos;
   C2POut& o = F.o;
+  KScF& k = L.k;
   o.err = ERR_RESET_ENTROPY;
   F.failed = true;
 #pragma unroll
@@ -1029,7 +1048,6 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
   pr[GRB_P_BX] = c[7]; pr[GRB_P_BY] = c[8]; pr[GRB_P_BZ] = c[9];
   F.lenient = m.alp < alp_bh_thresh;
   if (c[0] < 0) return F;  // c2p_back_f resets it to the atmosphere
-  KScF k;
   kscf<kBrent>(e, m, c, k);
   double ye = c[5] * k.iD;
   if (ye > e.yemax) { ye = e.yemax; o.err |= ERR_RESET_YE; }
@@ -1059,6 +1077,12 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
   }
   if (!(c[0] >= P.rho_fl * (1 + P.atmo_tol))) return F;
   F.ran = true;
+  if (!kDry) {
+    mvs(m.gi, c + 1, L.rup);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) L.rup[i] *= k.iD;
+    L.s = c[6] * k.iD;
+  }
   KFn f;
   f.e = &e;
   f.k = &k;
@@ -1084,6 +1108,7 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
   if (f.raw >= e.eps_max) F.ret |= SIG_EPS_HIGH;
   else if (f.raw < f.lo) F.ret |= SIG_EPS_LOW;
   F.failed = !(fabs(res) <= P.tol) || (F.ret & (SIG_RHO_HIGH | SIG_EPS_HIGH));
+  F.wb_ok = true;
   if (kDry) {
     // only rho, T, z^2 and b^2 decide whether the state is floored
     pr[GRB_P_RHO] = clamp_f(f.rho, e.rhomin, e.rhomax);
@@ -1091,15 +1116,10 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
     F.wb.z2 = f.w * f.w - 1.0;
     F.wb.Bz = f.w * mu * (k.rBt * (k.isD * k.D));
     F.wb.b2 = (k.b2 * k.D + F.wb.Bz * F.wb.Bz) * (f.iw * f.iw);
-    F.wb_ok = true;
     return F;
   }
-  take_solution(e, m, k, f, mu, c, pr, F.wb, F.wb_ok);
+  take_solution(e, L, f, mu, pr, F.wb, met);
   pr[GRB_P_ENT] = f.eth;
-  if (!F.wb_ok) {
-    F.wb = wb_of(m, pr);
-    F.wb_ok = true;
-  }
   const bool distrust =
       F.failed || (F.ret & SIG_EPS_LOW) || 2.0 * pr[GRB_P_PRESS] <= P.beta_fallback * fmax(F.wb.b2, 1e-50);
   F.backup = distrust && P.use_ent_backup;
@@ -1109,19 +1129,18 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
 // c2p_backup in the tuned mode.  The reference's solve clamps the entropy to
 // its range at every density it visits and keeps it clamped: the range at
 // the bracket's two ends, its largest and smallest density, covers all.
-template <bool kBrent>
-GRB_HD void c2p_backup_f(C2PState& F, double c[10], double pr[13], const Met& m, const DevParams& P) {
+template <bool kBrent, class MetF>
+GRB_HD void c2p_backup_f(C2PState& F, const C2PLive& L, double pr[13], const DevParams& P, MetF&& met) {
   const DevEos& e = P.eos;
   const bool ideal = e.kind == GRB_EOS_IDEAL_GAS;
-  KScF k;
-  kscf<kBrent>(e, m, c, k);
+  const KScF& k = L.k;
   const double mu0 = F.mu0 > 0.0 ? F.mu0 : mu0_f(e, k);
   EFn f;
   f.e = &e;
   f.k = &k;
   f.g = ideal ? e.gm1 : e.gthm1;
   f.elo = ideal ? e.ent_min : e.entropy_min;
-  const double lD = log(k.D), s0 = c[6] * k.iD;
+  const double lD = log(k.D), s0 = L.s;
   f.sl = s0 + lD;
   // whether any density of the bracket may leave the entropy's range: the
   // thermal energy at rho = D, and a lower bound of it at D/W
@@ -1143,16 +1162,20 @@ GRB_HD void c2p_backup_f(C2PState& F, double c[10], double pr[13], const Met& m,
     F.ret = sig;
     F.failed = false;
     F.o.err |= ERR_ENT_BACKUP;
-    take_solution(e, m, k, f, mu, c, pr, F.wb, F.wb_ok);
+    take_solution(e, L, f, mu, pr, F.wb, met);
+    F.wb_ok = true;
     pr[GRB_P_ENT] = clamp ? f.sl - lD : s0;
     F.ent_ok = true;
   }
   // otherwise the Kastaun primitives stand, or the state is reset if that failed
 }
 
-// c2p_back in the tuned mode.
-template <bool kAllCons = true, bool kDry = false>
-GRB_HD void c2p_back_f(C2PState& F, double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph) {
+// c2p_back in the tuned mode.  excise: the state lies in the excised region.
+// kAllCons false: the returned cons hold only what the reset flags in o.err
+// ask for.
+template <bool kAllCons = true, bool kDry = false, class MetF>
+GRB_HD void c2p_back_f(C2PState& F, double c[10], double pr[13], double sqrtg, const DevParams& P, bool excise,
+                       MetF&& met) {
   const DevEos& e = P.eos;
   const bool ideal = e.kind == GRB_EOS_IDEAL_GAS;
   C2POut& o = F.o;
@@ -1163,7 +1186,6 @@ GRB_HD void c2p_back_f(C2PState& F, double c[10], double pr[13], const Met& m, c
     if (ideal && (ret & SIG_EPS_LOW)) o.floored = true;
     handle_sig(ret, F.lenient, o.err, o.fatal);
   }
-  const bool excise = P.excise_by_radius ? (r_sph <= P.r_ex) : (m.alp <= P.alp_ex);
   // which replacement of the primitives: 1 atmosphere, 2 temperature floor, 3 magnetisation
   int rep = 0;
   if (F.failed || excise || pr[GRB_P_RHO] < (1. + P.atmo_tol) * P.rho_fl) {
@@ -1183,13 +1205,13 @@ GRB_HD void c2p_back_f(C2PState& F, double c[10], double pr[13], const Met& m, c
   } else {  // limit_primitives (c2p.cpp:63-115)
     uint32_t s2 = 0;
     const double z2max = P.max_w * P.max_w - 1.;
-    if (!F.wb_ok) { wb = wb_of(m, pr); F.wb_ok = true; }
+    if (!F.wb_ok) { wb = wb_of(met(), pr); F.wb_ok = true; }
     if (wb.z2 >= z2max) {
       s2 |= SIG_VEL_HIGH;
       if (!kDry) {
-        const double zn = 0.99 * sqrt_f(z2max * rcp_f(wb.z2));
+        const double zn = 0.99 * sqrt(z2max / wb.z2);
         pr[GRB_P_ZX] *= zn; pr[GRB_P_ZY] *= zn; pr[GRB_P_ZZ] *= zn;
-        wb = wb_of(m, pr);
+        wb = wb_of(met(), pr);
       }
     }
     if (wb.b2 >= P.max_sigma * pr[GRB_P_RHO]) {
@@ -1214,15 +1236,10 @@ GRB_HD void c2p_back_f(C2PState& F, double c[10], double pr[13], const Met& m, c
     pr[GRB_P_ENT] = ideal ? log(eth) * e.igm1 - log(pr[GRB_P_RHO])
                           : log(fmax(eth, e.entropy_min)) * e.igthm1 - log(pr[GRB_P_RHO]);
   }
-  if (!F.wb_ok) wb = wb_of(m, pr);
-  o.W = wb.W;
-  o.iW = wb.iW;
   const uint32_t need = kAllCons ? ~0u : o.err;
-  const double D = pr[GRB_P_RHO] * wb.W;
-  c[0] = m.sqrtg * D;
-  c[6] = m.sqrtg * (pr[GRB_P_ENT] * D);
-  c[5] = c[0] * pr[GRB_P_YE];
-  if (need & (ERR_RESET_STILDE | ERR_RESET_TAU)) {
+  if (!F.wb_ok || (need & (ERR_RESET_STILDE | ERR_RESET_TAU))) {
+    const Met m = met();
+    if (!F.wb_ok) wb = wb_of(m, pr);
     double zl[3], Bl[3];
     mvs(m.g, pr + GRB_P_ZX, zl);
     mvs(m.g, pr + GRB_P_BX, Bl);
@@ -1231,22 +1248,40 @@ GRB_HD void c2p_back_f(C2PState& F, double c[10], double pr[13], const Met& m, c
     const double hW = rhoh * wb.W;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
-      c[1 + i] = m.sqrtg * (hW * zl[i] - wb.Bz * ((Bl[i] + wb.Bz * zl[i]) * wb.iW));
-    c[4] = m.sqrtg * (hW * wb.W - pstar - wb.Bz * wb.Bz - D);
+      c[1 + i] = sqrtg * (hW * zl[i] - wb.Bz * ((Bl[i] + wb.Bz * zl[i]) * wb.iW));
+    c[4] = sqrtg * (hW * wb.W - pstar - wb.Bz * wb.Bz - pr[GRB_P_RHO] * wb.W);
   }
+  o.W = wb.W;
+  o.iW = wb.iW;
+  const double D = pr[GRB_P_RHO] * wb.W;
+  c[0] = sqrtg * D;
+  c[6] = sqrtg * (pr[GRB_P_ENT] * D);
+  c[5] = c[0] * pr[GRB_P_YE];
+}
+
+// Whether conservs_to_prims excises the state.
+GRB_HD bool excised(const DevParams& P, double alp, double r_sph) {
+  return P.excise_by_radius ? (r_sph <= P.r_ex) : (alp <= P.alp_ex);
 }
 
 // The whole c2p in the tuned mode, and the FOFC flag's dry run.
-template <bool kAllCons = true>
-GRB_HD C2POut c2p_f(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph, double alp_bh_thresh) {
-  C2PState F = c2p_front_f<false>(c, pr, m, P, alp_bh_thresh);
-  if (F.backup) c2p_backup_f<false>(F, c, pr, m, P);
-  c2p_back_f<kAllCons>(F, c, pr, m, P, r_sph);
+template <bool kAllCons, class MetF>
+GRB_HD C2POut c2p_f(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph, double alp_bh_thresh,
+                    MetF&& met) {
+  C2PLive L;
+  const bool ex = excised(P, m.alp, r_sph);
+  const double sqrtg = m.sqrtg;
+  C2PState F = c2p_front_f<false>(c, pr, m, P, alp_bh_thresh, L, met);
+  if (F.backup) c2p_backup_f<false>(F, L, pr, P, met);
+  c2p_back_f<kAllCons>(F, c, pr, sqrtg, P, ex, met);
   return F.o;
 }
-GRB_HD bool c2p_floored_f(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph) {
-  C2PState F = c2p_front_f<false, true>(c, pr, m, P, 1e30);
-  if (!F.done) c2p_back_f<true, true>(F, c, pr, m, P, r_sph);
+template <class MetF>
+GRB_HD bool c2p_floored_f(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph, MetF&& met) {
+  C2PLive L;
+  const bool ex = excised(P, m.alp, r_sph);
+  C2PState F = c2p_front_f<false, true>(c, pr, m, P, 1e30, L, met);
+  if (!F.done) c2p_back_f<true, true>(F, c, pr, 0.0, P, ex, met);
   return F.o.floored;
 }
 

@@ -319,6 +319,12 @@ __device__ __forceinline__ Met batch_metric(const double* __restrict__ metric, i
   return make_met<FAST>(g, b, alp);
 }
 
+// The same again, out of line: for the few states whose c2p needs the metric
+// after its root solve.
+__device__ __noinline__ Met batch_metric_again(const double* metric, int64_t n, int64_t t) {
+  return batch_metric<true>(metric, n, t);
+}
+
 // ---- batched c2p, plain or with the learned bracket ------------------------
 struct C2PDiagDev {
   int32_t* iters;      // Brent iterations
@@ -417,7 +423,13 @@ struct C2PDeferred {
   int64_t t;
 };
 
-template <bool kLearned>
+//
+// kDefer false: a batch of at most kC2PDirect states (two warps a scheduler)
+// runs the backups in place: with the GPU mostly empty there is nothing to
+// compact, and the second launch, its wait for the first and the cleared
+// count cost more than divergent warps.
+constexpr int64_t kC2PDirect = 148 * 2 * kC2PThreads;
+template <bool kLearned, bool kDefer = true>
 __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, int64_t n,
                                                                 const double* __restrict__ cons,
                                                                 const double* __restrict__ metric,
@@ -457,15 +469,18 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, in
     gs = mlp_bracket(S.net.nrm, out, mu0);
   }
   C2PState F{};
-  if (active)
+  const auto met = [&] { return batch_metric_again(metric, n, ts); };
+  C2PLive L;
+  if (active) {
     F = kLearned ? c2p_front<true>(c, pr, m, P, false, P.alp_bh_thresh, gs)
-                 : c2p_front_f<true>(c, pr, m, P, P.alp_bh_thresh);
-  const bool later = active && !F.done && F.backup;
+                 : c2p_front_f<true>(c, pr, m, P, P.alp_bh_thresh, L, met);
+  }
+  const bool later = kDefer && active && !F.done && F.backup;
   // one slot per deferred lane, one atomic per warp
   const unsigned mask = __ballot_sync(0xffffffffu, later);
   unsigned long long base = 0;
   const int lane = threadIdx.x & 31;
-  if (lane == 0 && mask) base = atomicAdd(ndefer, (unsigned long long)__popc(mask));
+  if (kDefer && lane == 0 && mask) base = atomicAdd(ndefer, (unsigned long long)__popc(mask));
   base = __shfl_sync(0xffffffffu, base, 0);
   if (!active) return;
   if (diag.iters) diag.iters[t] = F.o.iters;
@@ -485,7 +500,8 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, in
     d.t = t;
     return;
   }
-  if (!F.done) c2p_back_f(F, c, pr, m, P, 0.0);
+  if (!kDefer && F.backup) c2p_backup_f<true>(F, L, pr, P, met);
+  if (!F.done) c2p_back_f(F, c, pr, m.sqrtg, P, excised(P, m.alp, 0.0), met);
   if (F.o.fatal) atomicOr(flags, F.o.fatal);
   pr[GRB_P_CS2] = 0.0;
 #pragma unroll
@@ -517,8 +533,11 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_backup(DevParams P, i
     C2PState F = d.F;
     const int64_t t = d.t;
     const Met m = batch_metric<true>(metric, n, t);
-    c2p_backup_f<true>(F, c, pr, m, P);
-    c2p_back_f(F, c, pr, m, P, 0.0);
+    const auto met = [&] { return batch_metric_again(metric, n, t); };
+    C2PLive L;
+    c2p_live<true>(P.eos, m, c, L);
+    c2p_backup_f<true>(F, L, pr, P, met);
+    c2p_back_f(F, c, pr, m.sqrtg, P, excised(P, m.alp, 0.0), met);
     if (F.o.fatal) atomicOr(flags, F.o.fatal);
     pr[GRB_P_CS2] = 0.0;
 #pragma unroll

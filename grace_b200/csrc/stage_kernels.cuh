@@ -485,6 +485,16 @@ __device__ __forceinline__ Met cell_met(const Geo& G, const double* st, int i, i
   for (int a = 0; a < 3; ++a) b[a] = st[c0 + G.cells * (GRB_BETAX + a)];
   return make_met<FAST>(g, b, st[c0 + G.cells * GRB_ALP]);
 }
+// cell_met<true> of the cell with variable 0 at p, out of line: for the few
+// cells whose c2p needs the metric after its root solve.
+__device__ __noinline__ Met cell_met_again(const double* p, int64_t cells) {
+  double g[6], b[3];
+#pragma unroll
+  for (int a = 0; a < 6; ++a) g[a] = p[cells * (GRB_GXX + a)];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) b[a] = p[cells * (GRB_BETAX + a)];
+  return make_met<true>(g, b, p[cells * GRB_ALP]);
+}
 __device__ __forceinline__ double cell_r(const Geo& G, const double* coords, const double* ix, int i,
                                          int j, int k, int64_t q) {
   if (!coords) return 0.0;
@@ -581,7 +591,9 @@ __device__ __forceinline__ void fofc_flag_cell(const DevParams& P, const Geo& G,
     const Met m = cell_met<kFast>(G, os, i, j, k, q);
     double pr[13];
     const double r = cell_r(G, coords, ix, i, j, k, q);
-    floored = kFast ? c2p_floored_f(c, pr, m, P, r) : c2p_floored(c, pr, m, P, r);
+    const double* o0 = os + cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
+    floored = kFast ? c2p_floored_f(c, pr, m, P, r, [&] { return cell_met_again(o0, G.cells); })
+                    : c2p_floored(c, pr, m, P, r);
   }
   if (floored || dmp) {
     int8_t* T = B.ftag;
@@ -1018,12 +1030,16 @@ __device__ __forceinline__ Met aux_load(const Geo& G, int i, int j, int k, int64
   }
   return m;
 }
-// After the c2p: c, pr the c2p's output; cB the cell's densitized B.
+// After the c2p: c, pr the c2p's output; m the cell's metric (plain mode; the
+// tuned mode reloads the lapse and shift, which nothing in the c2p keeps
+// live, and the face B).
 template <bool kDt, bool kFast>
 __device__ __forceinline__ double aux_finish(const DevParams& P, const Geo& G, int i, int j, int k, int64_t q,
-                                             double* __restrict__ st, double* __restrict__ aux, const Met& m,
-                                             const double cB[3], const double c[10], const double pr[13],
-                                             const C2POut& o, const StageBufs& B, const DtArgs& dta) {
+                                             double* __restrict__ st, const double* __restrict__ bx,
+                                             const double* __restrict__ by, const double* __restrict__ bz,
+                                             double* __restrict__ aux, const Met& m, const double c[10],
+                                             const double pr[13], const C2POut& o, const StageBufs& B,
+                                             const DtArgs& dta) {
   double dtc = INFINITY;
   const int64_t c0 = cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
   const int64_t a0 = cvar(G, i, j, k, 0, GRB_N_AUX_VARS, q);
@@ -1051,18 +1067,23 @@ __device__ __forceinline__ double aux_finish(const DevParams& P, const Geo& G, i
     aux[a0 + G.cells * GRB_C2P_ERR] = (double)(prev | (uint64_t)o.err);
   }
   if (P.emf == GRB_EMF_GS) {
+    const double cB[3] = {0.5 * (bx[bxi(G, i, j, k, q)] + bx[bxi(G, i + 1, j, k, q)]),
+                          0.5 * (by[byi(G, i, j, k, q)] + by[byi(G, i, j + 1, k, q)]),
+                          0.5 * (bz[bzi(G, i, j, k, q)] + bz[bzi(G, i, j, k + 1, q)])};
     // tuned mode: 1/W of the final primitives from the c2p
     const double W = kFast ? o.W : sqrt(1. + sqs(m.g, pr + GRB_P_ZX));
+    const double alp = kFast ? st[c0 + G.cells * GRB_ALP] : m.alp;
     double vt[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a)
-      vt[a] = (kFast ? m.alp * pr[GRB_P_ZX + a] * o.iW : m.alp * pr[GRB_P_ZX + a] / W) - m.beta[a];
+      vt[a] = (kFast ? alp * pr[GRB_P_ZX + a] * o.iW : alp * pr[GRB_P_ZX + a] / W) -
+              (kFast ? st[c0 + G.cells * (GRB_BETAX + a)] : m.beta[a]);
     B.ecenter[eci(G, i, j, k, 0, q)] = cB[1] * vt[2] - cB[2] * vt[1];
     B.ecenter[eci(G, i, j, k, 1, q)] = -cB[0] * vt[2] + cB[2] * vt[0];
     B.ecenter[eci(G, i, j, k, 2, q)] = cB[0] * vt[1] - cB[1] * vt[0];
   }
   if (kDt && i >= G.g && i < G.nx + G.g && j >= G.g && j < G.ny + G.g && k >= G.g && k < G.nz + G.g)
-    dtc = dta.cfl / max_eigenspeed(P.eos, m, pr) * dta.dx[3 * q];
+    dtc = dta.cfl / max_eigenspeed(P.eos, kFast ? cell_met(G, st, i, j, k, q) : m, pr) * dta.dx[3 * q];
   return dtc;
 }
 
@@ -1075,11 +1096,15 @@ __device__ __forceinline__ double aux_cell(const DevParams& P, const Geo& G, int
                                            const DtArgs& dta) {
   double c[10], pr[13];
   const Met m = aux_load<kFast>(G, i, j, k, q, st, bx, by, bz, aux, idx, true, c);
-  const double cB[3] = {c[7], c[8], c[9]};
   const double r = cell_r(G, coords, idx + 3 * q, i, j, k, q);
-  const C2POut o = kFast ? c2p_f<false>(c, pr, m, P, r, P.alp_bh_thresh)
-                         : c2p(c, pr, m, P, r, false, P.alp_bh_thresh, no_guess());
-  return aux_finish<kDt, kFast>(P, G, i, j, k, q, st, aux, m, cB, c, pr, o, B, dta);
+  C2POut o;
+  if (kFast) {
+    const double* s0 = st + cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
+    o = c2p_f<false>(c, pr, m, P, r, P.alp_bh_thresh, [&] { return cell_met_again(s0, G.cells); });
+  } else {
+    o = c2p(c, pr, m, P, r, false, P.alp_bh_thresh, no_guess());
+  }
+  return aux_finish<kDt, kFast>(P, G, i, j, k, q, st, bx, by, bz, aux, m, c, pr, o, B, dta);
 }
 
 // The aux pass with the entropy backups deferred (tuned candidate, for
@@ -1162,15 +1187,17 @@ __global__ void __launch_bounds__(128, MINB) k_aux_front(DevParams P, Geo G, Box
   double dtc = INFINITY;
   const bool active = decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q);
   Met m;
-  double c[10], pr[13], cB[3];
+  double c[10], pr[13];
+  C2PLive L;
+  bool ex = false;
+  const double* s0 = nullptr;
   C2PState F{};
-  double r = 0.0;
+  const auto met = [&] { return cell_met_again(s0, G.cells); };
   if (active) {
     m = aux_load<true>(G, i, j, k, q, st, bx, by, bz, aux, idx, true, c);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) cB[a] = c[7 + a];
-    r = cell_r(G, coords, idx + 3 * q, i, j, k, q);
-    F = c2p_front_f<false>(c, pr, m, P, P.alp_bh_thresh);
+    s0 = st + cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
+    ex = excised(P, m.alp, cell_r(G, coords, idx + 3 * q, i, j, k, q));
+    F = c2p_front_f<false>(c, pr, m, P, P.alp_bh_thresh, L, met);
   }
   const bool later = active && F.backup;
   const unsigned mask = __ballot_sync(0xffffffffu, later);
@@ -1189,9 +1216,9 @@ __global__ void __launch_bounds__(128, MINB) k_aux_front(DevParams P, Geo G, Box
       d.F = F;
       d.i = i; d.j = j; d.k = k; d.q = q;
     } else {
-      if (F.backup) c2p_backup_f<false>(F, c, pr, m, P);
-      c2p_back_f<false>(F, c, pr, m, P, r);
-      dtc = aux_finish<kDt, true>(P, G, i, j, k, q, st, aux, m, cB, c, pr, F.o, B, dta);
+      if (F.backup) c2p_backup_f<false>(F, L, pr, P, met);
+      c2p_back_f<false>(F, c, pr, m.sqrtg, P, ex, met);
+      dtc = aux_finish<kDt, true>(P, G, i, j, k, q, st, bx, by, bz, aux, m, c, pr, F.o, B, dta);
     }
   }
   if (kDt) dt_reduce(dtc, dta.out);
@@ -1213,15 +1240,18 @@ __global__ void __launch_bounds__(128, MINB) k_aux_backup(DevParams P, Geo G, do
     const int64_t q = d.q;
     double c[10], pr[13];
     const Met m = aux_load<true>(G, i, j, k, q, st, bx, by, bz, aux, idx, false, c);
-    const double cB[3] = {c[7], c[8], c[9]};
+    const double* s0 = st + cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
+    const auto met = [&] { return cell_met_again(s0, G.cells); };
 #pragma unroll
     for (int v = 0; v < 10; ++v) c[v] = d.c[v];
 #pragma unroll
     for (int v = 0; v < 13; ++v) pr[v] = d.pr[v];
     C2PState F = d.F;
-    c2p_backup_f<false>(F, c, pr, m, P);
-    c2p_back_f<false>(F, c, pr, m, P, cell_r(G, coords, idx + 3 * q, i, j, k, q));
-    dtc = fmin(dtc, aux_finish<kDt, true>(P, G, i, j, k, q, st, aux, m, cB, c, pr, F.o, B, dta));
+    C2PLive L;
+    c2p_live<false>(P.eos, m, c, L);
+    c2p_backup_f<false>(F, L, pr, P, met);
+    c2p_back_f<false>(F, c, pr, m.sqrtg, P, excised(P, m.alp, cell_r(G, coords, idx + 3 * q, i, j, k, q)), met);
+    dtc = fmin(dtc, aux_finish<kDt, true>(P, G, i, j, k, q, st, bx, by, bz, aux, m, c, pr, F.o, B, dta));
   }
   if (kDt) dt_reduce(dtc, dta.out);
 }
