@@ -114,50 +114,69 @@ __global__ void __launch_bounds__(128) k_restrict_cells(Geo G, Box box, Restrict
 // coarse cells (k_restrict_lag_zcol) repeats each x contraction for the up
 // to three columns that share it and was bound by its 25 loads a plane.  512
 // blocks of 16^3, restricted and prolonged (23 variables, face B, three
-// element kinds): 514 us by columns, 429 us with this and k_prolong_lag.  The
+// element kinds): 514 us by columns, 396 us with this and k_prolong_lag
+// (restriction 170 / 113 us, prolongation of the 16 variables 166 / 99 us);
+// with the indices decoded per item, 81 instructions around 9 FP64 ones, 429.
+// The
 // operands and their order are lagrange_restrict_op<4>'s: x, y, z.
-// dx, dy: divisors nx/2 and ny (pass x), dz: ny/2.
-__global__ void __launch_bounds__(128) k_restrict_lag(Geo G, RestrictVars V, FastDiv dnv, FastDiv dx, FastDiv dy,
-                                                      FastDiv dz, const double* __restrict__ src,
-                                                      double* __restrict__ dst, const int64_t* __restrict__ src_q,
+__global__ void __launch_bounds__(128) k_restrict_lag(Geo G, RestrictVars V, FastDiv dnv,
+                                                      const double* __restrict__ src, double* __restrict__ dst,
+                                                      const int64_t* __restrict__ src_q,
                                                       const int64_t* __restrict__ dst_q,
                                                       const uint8_t* __restrict__ child) {
   extern __shared__ __align__(16) double sm_fmr[];
   const uint32_t iq = fast_div(blockIdx.x, dnv);
   const int v = list_var(V, (int)(blockIdx.x - iq * (uint32_t)V.n));
   const int N0 = G.NX, N1 = G.NY, g = G.g;
-  const int hx = G.nx / 2, hy = G.ny / 2, hz = G.nz / 2;
+  const int hx = G.nx / 2, hy = G.ny / 2, hz = G.nz / 2, np = hx * hy;
   const double* u = src + (src_q[iq] * GRB_N_EVOL_VARS + v) * G.cells;
   double* o = dst + (dst_q[iq] * GRB_N_EVOL_VARS + v) * G.cells;
   const uint8_t cid = child[iq];
+  const int tid = threadIdx.x;
   double* X = sm_fmr;                  // [nz][ny][hx]
   double* Y = X + hx * G.ny * G.nz;    // [nz][hy][hx]
-  for (int t = threadIdx.x; t < hx * G.ny * G.nz; t += 128) {
-    const uint32_t r = fast_div((uint32_t)t, dx), z = fast_div(r, dy);
-    const int i = t - (int)r * hx, y = (int)(r - z * (uint32_t)G.ny);
-    const int fi = 2 * i + g, ox = lag4_offset(fi, G.nx, g, cid & 1);
-    const double* l = u + ((int64_t)((int)z + g) * N1 + (y + g)) * N0 + fi + ox - 3;
-    const double line[5] = {l[0], l[1], l[2], l[3], l[4]};
-    X[t] = contract5_rn(c_restrict5 + 5 * ox, line);
+  // x: a thread keeps its column i (and so its weights) and walks the rows
+  for (int i = tid % hx, i0 = tid / hx; i < hx && i0 < 128 / hx; i += hx) {
+    const int fi = 2 * i + g, ox = lag4_offset(fi, G.nx, g, cid & 1), rows = 128 / hx;
+    double cf[5];
+#pragma unroll
+    for (int d = 0; d < 5; ++d) cf[d] = c_restrict5[5 * ox + d];
+    const double* l0 = u + fi + ox - 3 + ((int64_t)g * N1 + g) * N0;
+    int y = i0, z = 0;
+    while (y >= G.ny) { y -= G.ny; ++z; }
+    while (z < G.nz) {
+      const double* l = l0 + ((int64_t)z * N1 + y) * N0;
+      const double line[5] = {l[0], l[1], l[2], l[3], l[4]};
+      X[(z * G.ny + y) * hx + i] = contract5_rn(cf, line);
+      y += rows;
+      while (y >= G.ny) { y -= G.ny; ++z; }
+    }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < hx * hy * G.nz; t += 128) {
-    const uint32_t r = fast_div((uint32_t)t, dx), z = fast_div(r, dz);
-    const int i = t - (int)r * hx, j = (int)(r - z * (uint32_t)hy);
+  // y, z: a thread keeps its column (i, j) and walks along z, in 128 / np
+  // interleaved parts where the columns are fewer than the threads
+  const int parts = np < 128 ? 128 / np : 1, part = np < 128 ? tid / np : 0;
+  for (int ij = np < 128 ? tid % np : tid; ij < np && part < parts; ij += 128) {
+    const int j = ij / hx, i = ij - j * hx;
     const int fj = 2 * j + g, oy = lag4_offset(fj, G.ny, g, (cid >> 1) & 1);
-    const double* l = X + ((int)z * G.ny + 2 * j + oy - 3) * hx + i;
-    const double line[5] = {l[0], l[hx], l[2 * hx], l[3 * hx], l[4 * hx]};
-    Y[t] = contract5_rn(c_restrict5 + 5 * oy, line);
+    double cf[5];
+#pragma unroll
+    for (int d = 0; d < 5; ++d) cf[d] = c_restrict5[5 * oy + d];
+    for (int z = part; z < G.nz; z += parts) {
+      const double* l = X + (z * G.ny + 2 * j + oy - 3) * hx + i;
+      const double line[5] = {l[0], l[hx], l[2 * hx], l[3 * hx], l[4 * hx]};
+      Y[z * np + ij] = contract5_rn(cf, line);
+    }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < hx * hy * hz; t += 128) {
-    const uint32_t r = fast_div((uint32_t)t, dx), kz = fast_div(r, dz);
-    const int i = t - (int)r * hx, j = (int)(r - kz * (uint32_t)hy), k = (int)kz;
-    const int oz = lag4_offset(2 * k + g, G.nz, g, (cid >> 2) & 1);
-    const int s = hx * hy;
-    const double* l = Y + (2 * k + oz - 3) * s + j * hx + i;
-    const double line[5] = {l[0], l[s], l[2 * s], l[3 * s], l[4 * s]};
-    o[((int64_t)(k + g) * N1 + (j + g)) * N0 + (i + g)] = contract5_rn(c_restrict5 + 5 * oz, line);
+  for (int ij = np < 128 ? tid % np : tid; ij < np && part < parts; ij += 128) {
+    const int j = ij / hx, i = ij - j * hx;
+    for (int k = part; k < hz; k += parts) {
+      const int oz = lag4_offset(2 * k + g, G.nz, g, (cid >> 2) & 1);
+      const double* l = Y + (2 * k + oz - 3) * np + ij;
+      const double line[5] = {l[0], l[np], l[2 * np], l[3 * np], l[4 * np]};
+      o[((int64_t)(k + g) * N1 + (j + g)) * N0 + (i + g)] = contract5_rn(c_restrict5 + 5 * oz, line);
+    }
   }
 }
 
@@ -360,9 +379,12 @@ __global__ void __launch_bounds__(256) k_prolong_lag(Geo G, RestrictVars V, Fast
                                                      const int64_t* __restrict__ cbuf_q,
                                                      const uint8_t* __restrict__ elem) {
   extern __shared__ __align__(16) double sm_fmr[];
+  __shared__ int64_t voff[kV];  // the CTA's variables, as offsets
   const uint32_t iq = fast_div(blockIdx.x, dgroups);
   const int v0 = (int)(blockIdx.x - iq * dgroups.d) * kV;
   const int nv = min(kV, V.n - v0);
+  if (threadIdx.x < nv) voff[threadIdx.x] = list_var(V, v0 + (int)threadIdx.x) * G.cells;
+  __syncthreads();
   const int e = elem[iq], n = G.nx, g = G.g;
   int r[3], k0[3], f0[3];
   bool along[3];
@@ -387,7 +409,7 @@ __global__ void __launch_bounds__(256) k_prolong_lag(Geo G, RestrictVars V, Fast
   for (int t = threadIdx.x; t < nv * wz * wy * r[0]; t += 256) {
     const uint32_t a = fast_div((uint32_t)t, drx), b = fast_div(a, dwy), c = fast_div(b, dwz);
     const int x = t - (int)a * r[0], y = (int)(a - b * (uint32_t)wy), z = (int)(b - c * (uint32_t)wz);
-    const double* l = ub + list_var(V, v0 + (int)c) * G.cells +
+    const double* l = ub + voff[c] +
                       ((int64_t)(k0[2] + z - 2) * N1 + (k0[1] + y - 2)) * N0 + k0[0] + x - 2;
     const double line[5] = {l[0], l[1], l[2], l[3], l[4]};
     double* s = X + (int)a * fx + 2 * x;
@@ -411,7 +433,7 @@ __global__ void __launch_bounds__(256) k_prolong_lag(Geo G, RestrictVars V, Fast
     const int s = fx * fy;
     const double* l = Y + ((int)c * wz + z) * s + y * fx + x;
     const double line[5] = {l[0], l[s], l[2 * s], l[3 * s], l[4 * s]};
-    double* o = ob + list_var(V, v0 + (int)c) * G.cells + ((int64_t)(f0[2] + 2 * z) * N1 + (f0[1] + y)) * N0 + f0[0] + x;
+    double* o = ob + voff[c] + ((int64_t)(f0[2] + 2 * z) * N1 + (f0[1] + y)) * N0 + f0[0] + x;
     o[0] = contract5_rn(c_prolong5, line);
     o[(int64_t)N1 * N0] = contract5_rn(c_prolong5 + 5, line);
   }

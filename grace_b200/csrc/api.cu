@@ -291,7 +291,7 @@ template <int dir, int MINB, int NT = 128>
 bool launch_flux_tma(cudaStream_t s, const DevParams& P, const Geo& G, const Box& b, const double* st,
                      const double* aux, const double* bf, const StageBufs& B) {
   const FluxTile T = flux_tile(dir, G, b, NT);
-  if (T.n[0] > NT || b.nq > 65535) return false;
+  if (T.R < 1 || b.nq > 65535) return false;
   CUtensorMap ta, tm;
   if (!make_tmap(&ta, aux, G, GRB_N_AUX_VARS, b.nq, T) || !make_tmap(&tm, st, G, GRB_N_EVOL_VARS, b.nq, T))
     return false;
@@ -328,7 +328,7 @@ bool launch_flux_tma3(cudaStream_t s, const DevParams& P, const Geo& G, const do
   for (int d = 0; d < 3; ++d) {
     const Box b = face_box(G, P.emf, d, G.nq);
     A.T[d] = flux_tile(d, G, b, NT);
-    if (A.T[d].n[0] > NT || b.nq > 65535) return false;
+    if (A.T[d].R < 1 || b.nq > 65535) return false;
     if (!make_tmap(&A.aux[d], aux, G, GRB_N_AUX_VARS, b.nq, A.T[d]) ||
         !make_tmap(&A.met[d], st, G, GRB_N_EVOL_VARS, b.nq, A.T[d]))
       return false;
@@ -381,7 +381,7 @@ template <int dir, int MINB, int NT = 128>
 bool launch_flux_tma_queue(cudaStream_t s, const DevParams& P, const Geo& G, const Box& b, const double* st,
                            const double* aux, const double* bf, const StageBufs& B, unsigned long long* queue) {
   const FluxTile T = flux_tile(dir, G, b, NT);
-  if (T.n[0] > NT || !queue) return false;
+  if (T.R < 1 || !queue) return false;
   CUtensorMap ta, tm;
   if (!make_tmap(&ta, aux, G, GRB_N_AUX_VARS, b.nq, T) || !make_tmap(&tm, st, G, GRB_N_EVOL_VARS, b.nq, T))
     return false;
@@ -962,7 +962,7 @@ int grb_reserve(grb_handle* h, const grb_grid* g) {
     // the compacted FOFC face list: up to 4 Mi faces a substep (more falls
     // back to the full recompute launch)
     h->B.fcap = h->fcap_alloc = (uint32_t)std::min<int64_t>(nf * 3, 1 << 22);
-    ok = al((void**)&h->B.flist, sizeof(uint32_t) * h->B.fcap) && al((void**)&h->B.fcount, sizeof(uint32_t));
+    ok = al((void**)&h->B.flist, sizeof(uint32_t) * h->B.fcap) && al((void**)&h->B.fcount, 2 * sizeof(uint32_t));
   }
   if (!ok) {
     free_scratch(h);
@@ -2061,11 +2061,10 @@ int grb_restrict_to_coarse(grb_handle* h, const grb_grid* g, const grb_fields* f
       const size_t smem = sizeof(double) * ((size_t)G.nx / 2 * G.ny * G.nz + (size_t)G.nx / 2 * (G.ny / 2) * G.nz);
       // below 6 cells along y or z the stencils reach ghost cells, which the
       // staged interior does not hold
-      if (G.ny >= 6 && G.nz >= 6 && smem <= kFmrSmem && (int64_t)nl * nquads <= 0x7fffffff &&
+      if (G.nx <= 256 && G.ny >= 6 && G.nz >= 6 && smem <= kFmrSmem && (int64_t)nl * nquads <= 0x7fffffff &&
           fmr_smem(k_restrict_lag)) {
         k_restrict_lag<<<(unsigned)(nl * nquads), 128, smem, s>>>(
-            G, V, make_fastdiv((uint32_t)nl), make_fastdiv((uint32_t)G.nx / 2), make_fastdiv((uint32_t)G.ny),
-            make_fastdiv((uint32_t)G.ny / 2), fine->state, cbuf->state, src_q, dst_q, child_id);
+            G, V, make_fastdiv((uint32_t)nl), fine->state, cbuf->state, src_q, dst_q, child_id);
       } else if (G.nz < 6) {
         // with 4 cells along z the edge stencils' windows move back along z
         k_restrict_cells<true><<<nblk(b.count(), 128), 128, 0, s>>>(G, b, V, make_fastdiv((uint32_t)nl), fine->state,

@@ -30,7 +30,9 @@ struct StageBufs {
   unsigned long long* nadefer = nullptr;
   int64_t adefer_cap = 0;
   // compacted list of the tagged faces (tuned mode): entries t << 2 | dir
-  // (t the FOFC box index), *fcount of them, room for fcap
+  // (t the FOFC box index), fcount[0] of them, room for fcap; fcount[1] is
+  // nonzero when the stage tagged anything (the passes over the tags return
+  // at once otherwise: most stages of a smooth flow)
   uint32_t* flist = nullptr;
   uint32_t* fcount = nullptr;
   uint32_t fcap = 0;
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(128) k_emf_gs(Geo G, Box box, StageBufs B, boo
   int64_t q;
   if (zero && blockIdx.x == 0 && threadIdx.x == 0) {
     B.counters[0] = B.counters[1] = 0;
-    if (B.fcount) *B.fcount = 0;
+    if (B.fcount) B.fcount[0] = B.fcount[1] = 0;
   }
   if (!decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q)) return;
   if (i < G.nx + G.g) B.emf[emi(G, i, j, k, 0, q)] = gs_edge(G, B, 0, i, j, k, q);
@@ -596,6 +598,7 @@ __device__ __forceinline__ void fofc_flag_cell(const DevParams& P, const Geo& G,
                     : c2p_floored(c, pr, m, P, r);
   }
   if (floored || dmp) {
+    if (B.fcount) B.fcount[1] = 1;
     int8_t* T = B.ftag;
     T[emi(G, i, j, k, 0, q)] = 1; T[emi(G, i + 1, j, k, 0, q)] = 1;
     T[emi(G, i, j, k, 1, q)] = 1; T[emi(G, i, j + 1, k, 1, q)] = 1;
@@ -664,6 +667,7 @@ __global__ void __launch_bounds__(128) k_fofc_faces(DevParams P, Geo G, Box box,
                                                      const double* __restrict__ bx,
                                                      const double* __restrict__ by,
                                                      const double* __restrict__ bz, StageBufs B) {
+  if (B.fcount && B.fcount[1] == 0) return;
   int i, j, k;
   int64_t q;
   if (!decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q)) return;
@@ -693,6 +697,7 @@ __global__ void __launch_bounds__(128) k_fofc_faces(DevParams P, Geo G, Box box,
 // count still grows, which sends k_fofc_faces_list to its whole-box loop.
 // Needs box.count() < 2^30.
 __global__ void __launch_bounds__(256) k_fofc_scan(Geo G, Box box, StageBufs B) {
+  if (B.fcount[1] == 0) return;
   int i, j, k;
   int64_t q;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -777,6 +782,7 @@ __global__ void __launch_bounds__(128) k_fofc_faces_list(DevParams P, Geo G, Box
   }
 }
 __global__ void __launch_bounds__(128) k_fofc_edges(Geo G, Box box, StageBufs B) {
+  if (B.fcount && B.fcount[1] == 0) return;
   int i, j, k;
   int64_t q;
   if (!decode(box, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i, j, k, q)) return;
