@@ -263,7 +263,7 @@ Box face_box(const Geo& G, int emf, int dir, int64_t nq) {
 FluxTile flux_tile(int dir, const Geo& G, const Box& b, int nt) {
   FluxTile T;
   for (int a = 0; a < 3; ++a) { T.lo[a] = b.lo[a]; T.n[a] = b.n[a]; }
-  T.R = nt / T.n[0];
+  T.R = dir == 0 ? (nt / 32 * 31 + 1) / (T.n[0] + 1) : nt / T.n[0];
   T.BY = dir == 0 ? T.R : dir == 1 ? T.R + 5 : 1;
   T.BZ = dir == 2 ? T.R + 5 : 1;
   (void)G;

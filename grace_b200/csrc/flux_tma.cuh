@@ -53,15 +53,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, int li
   return false;
 }
 
-// getflux<dir> on a staged stencil.  A, M: aux / metric tile at stencil
-// cell 0 (the cell three before the face) of variable 0; vs: variable
-// stride; st: stencil stride (cells along dir).
+// The r-th reconstructed variable: its aux index, its place in the primitives.
+__host__ __device__ constexpr int tile_var(int r) {
+  return r < 4 ? GRB_RHO + r : r == 4 ? GRB_YE : r == 5 ? GRB_TEMP : r == 6 ? GRB_ENTROPY : GRB_BX + r - 7;
+}
+__host__ __device__ constexpr int tile_prim(int r) {
+  return r == 0 ? GRB_P_RHO : r < 4 ? GRB_P_ZX + r - 1 : r == 4 ? GRB_P_YE : r == 5 ? GRB_P_TEMP : r == 6 ? GRB_P_ENT : GRB_P_BX + r - 7;
+}
+
+// getflux<dir> on a staged stencil after the reconstruction (pl, pr).  M:
+// metric tile at stencil cell 0 (the cell three before the face) of variable
+// 0; vs: variable stride; st: stencil stride (cells along dir).
 template <int dir>
-__device__ __forceinline__ void getflux_tile(const DevParams& P, int recon, bool rusanov, const double* A,
-                                             const double* M, int vs, int st, double bface, double f[7],
-                                             double vb[4]) {
-  const double alpl = M[(GRB_ALP - GRB_GXX) * vs + 2 * st];
-  const double alpr = M[(GRB_ALP - GRB_GXX) * vs + 3 * st];
+__device__ __forceinline__ void getflux_states(const DevParams& P, bool rusanov, const double* M, int vs, int st,
+                                               double bface, double* pl, double* pr, double f[7], double vb[4]) {
   double gm[10];
 #pragma unroll
   for (int a = 0; a < 10; ++a) {
@@ -69,29 +74,36 @@ __device__ __forceinline__ void getflux_tile(const DevParams& P, int recon, bool
     gm[a] = face4(p[st], p[2 * st], p[3 * st], p[4 * st]);
   }
   const Met m = make_met<true>(gm, gm + 7, gm[6]);
-  const int av[10] = {GRB_RHO, GRB_ZVECX, GRB_ZVECY, GRB_ZVECZ, GRB_YE, GRB_TEMP, GRB_ENTROPY, GRB_BX, GRB_BY, GRB_BZ};
-  const int pv[10] = {GRB_P_RHO, GRB_P_ZX, GRB_P_ZY, GRB_P_ZZ, GRB_P_YE, GRB_P_TEMP, GRB_P_ENT, GRB_P_BX, GRB_P_BY, GRB_P_BZ};
-  double pl[13], pr[13];
-  const bool donor = (alpl <= P.alp_ex || alpr <= P.alp_ex);
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const double* p = A + av[r] * vs;
-    if (donor) {
-      pl[pv[r]] = p[2 * st];
-      pr[pv[r]] = p[3 * st];
-    } else {
-      double u[6];
-#pragma unroll
-      for (int o = 0; o < 6; ++o) u[o] = p[o * st];
-      recon6_fast(recon, u, pl[pv[r]], pr[pv[r]]);
-    }
-  }
   const double bn = bface * m.isqrtg;
   pl[GRB_P_BX + dir] = bn;
   pr[GRB_P_BX + dir] = bn;
   eos_PT_f(P.eos, pl);
   eos_PT_f(P.eos, pr);
   mhd_fluxes_f<dir>(P, rusanov, pl, pr, m, f, vb);
+}
+// Both with the reconstruction; A: aux tile at stencil cell 0.
+template <int dir>
+__device__ __forceinline__ void getflux_tile(const DevParams& P, int recon, bool rusanov, const double* A,
+                                             const double* M, int vs, int st, double bface, double f[7],
+                                             double vb[4]) {
+  const double alpl = M[(GRB_ALP - GRB_GXX) * vs + 2 * st];
+  const double alpr = M[(GRB_ALP - GRB_GXX) * vs + 3 * st];
+  double pl[13], pr[13];
+  const bool donor = (alpl <= P.alp_ex || alpr <= P.alp_ex);
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    const double* p = A + tile_var(r) * vs;
+    if (donor) {
+      pl[tile_prim(r)] = p[2 * st];
+      pr[tile_prim(r)] = p[3 * st];
+    } else {
+      double u[6];
+#pragma unroll
+      for (int o = 0; o < 6; ++o) u[o] = p[o * st];
+      recon6_fast(recon, u, pl[tile_prim(r)], pr[tile_prim(r)]);
+    }
+  }
+  getflux_states<dir>(P, rusanov, M, vs, st, bface, pl, pr, f, vb);
 }
 
 constexpr int kTmaWaitLimit = 1 << 22;
@@ -107,6 +119,63 @@ __host__ __device__ inline size_t flux_tile_smem(const Geo& G, const FluxTile& T
   return 2 * sizeof(double) * (size_t)flux_tile_doubles(G, T) + 16;
 }
 
+// The x faces of a staged tile.  A thread takes one cell: WENO-Z's states on
+// its two faces share their weights (weno_z_cell), and the left state of its
+// lower face comes from the lane below.  A row's n + 1 cells (the one below
+// the first face included) follow each other over the lanes, consecutive
+// warps overlapping by one cell, whose face the lower warp computes: 31 of 32
+// lanes and n of n + 1 cells have a face.  Along y and z the neighbour sits
+// in another warp, and passing the states through shared memory costs the
+// gain again, so those reconstruct per face.
+__device__ __forceinline__ void flux_tile_face_x(const DevParams& P, const Geo& G, const FluxTile& T,
+                                                 const double* sa, const double* sm, int vs, int oy, int oz,
+                                                 int64_t q, const double* __restrict__ bface, const StageBufs& B) {
+  const int lane = threadIdx.x & 31, W = T.n[0] + 1;
+  const int c = (threadIdx.x >> 5) * 31 + lane;
+  int r = c / W, x = c - r * W;
+  bool face = lane > 0 && x > 0 && r < T.R && oy + r < T.lo[1] + T.n[1];
+  if (r >= T.R) { r = 0; x = 1; }
+  const int i = T.lo[0] - 1 + x;
+  const int base = r * G.NX + i - 3;  // stencil cell 0 of face i
+  const double* A = sa + base;
+  double pl[13], pr[13];
+  if (P.recon == GRB_RECON_WENOZ) {
+#pragma unroll
+    for (int v = 0; v < 10; ++v) {
+      const double* p = A + tile_var(v) * vs + 1;
+      const double u[5] = {p[0], p[1], p[2], p[3], p[4]};
+      double hi;
+      weno_z_cell(u, pr[tile_prim(v)], hi);
+      pl[tile_prim(v)] = __shfl_up_sync(0xffffffffu, hi, 1);
+    }
+    if (!face) return;
+    if (sm[base + (GRB_ALP - GRB_GXX) * vs + 2] <= P.alp_ex || sm[base + (GRB_ALP - GRB_GXX) * vs + 3] <= P.alp_ex) {
+#pragma unroll
+      for (int v = 0; v < 10; ++v) {
+        pl[tile_prim(v)] = A[tile_var(v) * vs + 2];
+        pr[tile_prim(v)] = A[tile_var(v) * vs + 3];
+      }
+    }
+  } else {
+    if (!face) return;
+    const bool donor = sm[base + (GRB_ALP - GRB_GXX) * vs + 2] <= P.alp_ex ||
+                       sm[base + (GRB_ALP - GRB_GXX) * vs + 3] <= P.alp_ex;
+#pragma unroll
+    for (int v = 0; v < 10; ++v) {
+      const double* p = A + tile_var(v) * vs;
+      const double u[6] = {p[0], p[1], p[2], p[3], p[4], p[5]};
+      double ul, ur;
+      recon6_fast(P.recon, u, ul, ur);
+      pl[tile_prim(v)] = donor ? u[2] : ul;
+      pr[tile_prim(v)] = donor ? u[3] : ur;
+    }
+  }
+  double f[7], vb[4];
+  const int j = oy + r, k = oz;
+  getflux_states<0>(P, P.riemann == GRB_RIEMANN_LLF, sm + base, vs, 1, __ldg(bface + bxi(G, i, j, k, q)), pl, pr, f, vb);
+  store_face(G, B, P.emf, 0, i, j, k, q, f, vb);
+}
+
 // The face of this thread in a staged tile (box origin oy, oz of block q):
 // lanes along x, rows along the tile's row axis; threads past the tile's
 // faces do nothing.
@@ -114,34 +183,34 @@ template <int dir>
 __device__ __forceinline__ void flux_tile_face(const DevParams& P, const Geo& G, const FluxTile& T,
                                                const double* sa, const double* sm, int vs, int oy, int oz,
                                                int64_t q, const double* __restrict__ bface, const StageBufs& B) {
+  if (dir == 0) {
+    flux_tile_face_x(P, G, T, sa, sm, vs, oy, oz, q, bface, B);
+    return;
+  }
   const int W = T.n[0];
   const int w = threadIdx.x % W, r = threadIdx.x / W;
   if (r >= T.R) return;
   const int i = T.lo[0] + w;
-  int j, k, base, st;
-  if (dir == 0) {
-    j = oy + r; k = oz;
-    if (j >= T.lo[1] + T.n[1]) return;
-    base = r * G.NX + i - 3; st = 1;
-  } else if (dir == 1) {
+  int j, k;
+  if (dir == 1) {
     j = oy + 3 + r; k = oz;
     if (j >= T.lo[1] + T.n[1]) return;
-    base = r * G.NX + i; st = G.NX;
   } else {
     j = oy; k = oz + 3 + r;
     if (k >= T.lo[2] + T.n[2]) return;
-    base = r * G.NX + i; st = G.NX;
   }
-  const int64_t bi = dir == 0 ? bxi(G, i, j, k, q) : dir == 1 ? byi(G, i, j, k, q) : bzi(G, i, j, k, q);
+  const int base = r * G.NX + i, st = G.NX;
+  const int64_t bi = dir == 1 ? byi(G, i, j, k, q) : bzi(G, i, j, k, q);
   double f[7], vb[4];
   getflux_tile<dir>(P, P.recon, P.riemann == GRB_RIEMANN_LLF, sa + base, sm + base, vs, st, __ldg(bface + bi), f, vb);
   store_face(G, B, P.emf, dir, i, j, k, q, f, vb);
 }
 
 // grid: (ceil(n_row / R), n_other, nq); NT threads (128 or 256); W = n[0]
-// <= NT; R = NT / W rows (a 256-thread tile re-reads the 5-row stencil halo
-// of the y and z directions over twice as many rows).
-//   dir 0: lanes i (faces), rows j, other k; box rows j (BY = R, BZ = 1)
+// <= NT; R = NT / W rows, for dir 0 (31 NT / 32 + 1) / (W + 1) (a 256-thread
+// tile re-reads the 5-row stencil halo of the y and z directions over twice
+// as many rows).
+//   dir 0: lanes i (cells), rows j, other k; box rows j (BY = R, BZ = 1)
 //   dir 1: lanes i, rows j (faces), other k; box rows j - 3 .. (BY = R + 5)
 //   dir 2: lanes i, rows k (faces), other j; box rows k - 3 .. (BZ = R + 5)
 template <int dir>
