@@ -424,13 +424,16 @@ struct C2PDeferred {
 };
 
 //
+// 4 CTAs per SM (128 registers, at most 140 bytes of spills in the backup):
+// at 3, the uncapped 136 and 168 registers, 2 M states took 1008 us against
+// 873; the dependent chains of the solves want warps more than registers.
 // kDefer false: a batch of at most kC2PDirect states (two warps a scheduler)
 // runs the backups in place: with the GPU mostly empty there is nothing to
 // compact, and the second launch, its wait for the first and the cleared
 // count cost more than divergent warps.
 constexpr int64_t kC2PDirect = 148 * 2 * kC2PThreads;
 template <bool kLearned, bool kDefer = true>
-__global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, int64_t n,
+__global__ void __launch_bounds__(kC2PThreads, kDefer && !kLearned ? 4 : 1) k_c2p_batch_front(DevParams P, int64_t n,
                                                                 const double* __restrict__ cons,
                                                                 const double* __restrict__ metric,
                                                                 double* __restrict__ prims,
@@ -515,7 +518,7 @@ __global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_front(DevParams P, in
 
 // The listed states: the entropy backup and the rest of the policy
 // (grid-stride over the count the front kernel left).
-__global__ void __launch_bounds__(kC2PThreads) k_c2p_batch_backup(DevParams P, int64_t n,
+__global__ void __launch_bounds__(kC2PThreads, 4) k_c2p_batch_backup(DevParams P, int64_t n,
                                                                  const double* __restrict__ metric,
                                                                  double* __restrict__ prims,
                                                                  double* __restrict__ cons_out,
