@@ -712,9 +712,10 @@ struct KScF {
 template <bool kRound>
 GRB_HD void kscf(const DevEos& e, const Met& m, const double c[10], KScF& k) {
   k.D = c[0];
-  k.iD = kRound ? 1.0 / k.D : rcp_f(k.D);
+  const double Df = k.D > 1e300 ? 1e300 : k.D;  // rcp_f and rsqrt_f of infinity are NaN
+  k.iD = kRound ? 1.0 / k.D : rcp_f(Df);
   k.q = c[4] * k.iD;
-  const double isD = kRound ? 1.0 / sqrt(k.D) : rsqrt_f(k.D);
+  const double isD = kRound ? 1.0 / sqrt(k.D) : rsqrt_f(Df);
   double r[3], Bt[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) { r[i] = c[1 + i] * k.iD; Bt[i] = c[7 + i] * isD; }
@@ -1064,12 +1065,17 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
     o.floored = true;
   }
   const double qd = k.q + 1;
-  if (k.r2 > qd * qd) {
-    const double f = sqrt(qd * qd / k.r2);
-    c[1] *= f; c[2] *= f; c[3] *= f;
-    kscf<kBrent>(e, m, c, k);
-    o.err |= ERR_RESET_STILDE;
-    o.floored = true;
+  if (!(k.r2 <= qd * qd)) {
+    // S^2 / D^2 itself: r^i = S^i / D overflows before it, and infinite r^i
+    // leave r^2 undefined
+    const double st2 = sqs(m.gi, c + 1) * (k.iD * k.iD);
+    if (st2 > qd * qd) {
+      const double f = sqrt(qd * qd / st2);
+      c[1] *= f; c[2] *= f; c[3] *= f;
+      kscf<kBrent>(e, m, c, k);
+      o.err |= ERR_RESET_STILDE;
+      o.floored = true;
+    }
   }
   if (o.floored && kDry) {
     F.done = true;
@@ -1107,7 +1113,8 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
   else if (f.rho <= e.rhomin) F.ret |= SIG_RHO_LOW;
   if (f.raw >= e.eps_max) F.ret |= SIG_EPS_HIGH;
   else if (f.raw < f.lo) F.ret |= SIG_EPS_LOW;
-  F.failed = !(fabs(res) <= P.tol) || (F.ret & (SIG_RHO_HIGH | SIG_EPS_HIGH));
+  // (a NaN tau reaches f through the clamped eps alone, which hides it)
+  F.failed = !(fabs(res) <= P.tol) || !(f.raw == f.raw) || (F.ret & (SIG_RHO_HIGH | SIG_EPS_HIGH));
   F.wb_ok = true;
   if (kDry) {
     // only rho, T, z^2 and b^2 decide whether the state is floored
@@ -1152,7 +1159,8 @@ GRB_HD void c2p_backup_f(C2PState& F, const C2PLive& L, double pr[13], const Dev
   double res;
   const double mu = kBrent ? brent_root(f, mu0, clamp, it, res)
                            : secant_root(f, mu0, e.ih0 * (1 + 1e-10), clamp, it, res);
-  if (fabs(res) <= P.tol && f.eps < e.eps_max) {
+  // (the clamps of eth would let a NaN entropy pass)
+  if (s0 == s0 && fabs(res) <= P.tol && f.eps < e.eps_max) {
     uint32_t sig = 0;
     if (f.vhigh) sig |= SIG_VEL_HIGH;
     if (f.rho >= e.rhomax) sig |= SIG_RHO_HIGH;
