@@ -117,8 +117,7 @@ __global__ void __launch_bounds__(128) k_restrict_cells(Geo G, Box box, Restrict
 // element kinds): 514 us by columns, 396 us with this and k_prolong_lag
 // (restriction 170 / 113 us, prolongation of the 16 variables 166 / 99 us);
 // with the indices decoded per item, 81 instructions around 9 FP64 ones, 429.
-// The
-// operands and their order are lagrange_restrict_op<4>'s: x, y, z.
+// The operands and their order are lagrange_restrict_op<4>'s: x, y, z.
 __global__ void __launch_bounds__(128) k_restrict_lag(Geo G, RestrictVars V, FastDiv dnv,
                                                       const double* __restrict__ src, double* __restrict__ dst,
                                                       const int64_t* __restrict__ src_q,
@@ -181,7 +180,7 @@ __global__ void __launch_bounds__(128) k_restrict_lag(Geo G, RestrictVars V, Fas
 }
 
 // High-order list of blocks whose contractions do not fit shared memory
-// (interiors above 28^3), one thread per (i, j) column of coarse cells and
+// (interiors above 24^3), one thread per (i, j) column of coarse cells and
 // variable, walking the column along z: each fine plane's contractions along
 // x and y (with the column's x and y stencils) are computed once and the
 // last five kept in registers; coarse cell k takes the z contraction of the
@@ -190,7 +189,8 @@ __global__ void __launch_bounds__(128) k_restrict_lag(Geo G, RestrictVars V, Fas
 // edge and half-dependent offsets keep their ends non-decreasing), so one
 // pass over the fine planes ngz .. nz + ngz - 1 serves every cell.  The
 // operands and their order are those of k_restrict_lag, bit for bit.  512
-// blocks of 16^3, 16 variables: 170 us.  box: (nx/2, ny/2, 1) x (nvars_in_list x nquads), variable fastest.
+// blocks of 16^3, 16 variables: 170 us.  box: (nx/2, ny/2, 1) x
+// (nvars_in_list x nquads), variable fastest.
 __global__ void __launch_bounds__(128) k_restrict_lag_zcol(Geo G, Box box, RestrictVars V, FastDiv dnv,
                                                            const double* __restrict__ src, double* __restrict__ dst,
                                                            const int64_t* __restrict__ src_q,
