@@ -303,11 +303,13 @@ int grb_linop_apply3(grb_handle* h, const grb_grid* g, const grb_fields* A, cons
  *          state, the plain bracket when the learned one misses the root);
  *          GRB_ERR_NO_MODEL without a model.
  * GRB_MODE_TUNED evaluates the c2p with the tuned-mode arithmetic (the same
- * functions up to rounding: fewer divisions, W and b^2 formed once) and
- * defers the entropy-based backup solves to a second pass over the states
+ * functions up to rounding: fewer divisions, W and b^2 formed once).  Up to
+ * 37 888 states (two CTAs of 128 per SM) each thread finishes its state,
+ * nothing is allocated.  Larger batches, and every batch with use_learned,
+ * defer the entropy-based backup solves to a second pass over the states
  * that need them (compacted, so its warps are uniform; each state's
  * operations and their order unchanged).  The handle keeps one record per
- * state for that pass: the first tuned call with a larger n allocates it
+ * state for that pass: the first such call with a larger n allocates it
  * (make it before any stream capture). */
 int grb_c2p_batch(grb_handle* h, int64_t n, const double* cons,
                   const double* metric, double* prims, double* cons_out,
