@@ -321,7 +321,7 @@ __device__ __forceinline__ Met batch_metric(const double* __restrict__ metric, i
 
 // The same again, out of line: for the few states whose c2p needs the metric
 // after its root solve.
-__device__ __noinline__ Met batch_metric_again(const double* metric, int64_t n, int64_t t) {
+static __device__ __noinline__ Met batch_metric_again(const double* metric, int64_t n, int64_t t) {
   return batch_metric<true>(metric, n, t);
 }
 

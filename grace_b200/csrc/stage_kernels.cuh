@@ -489,7 +489,7 @@ __device__ __forceinline__ Met cell_met(const Geo& G, const double* st, int i, i
 }
 // cell_met<true> of the cell with variable 0 at p, out of line: for the few
 // cells whose c2p needs the metric after its root solve.
-__device__ __noinline__ Met cell_met_again(const double* p, int64_t cells) {
+static __device__ __noinline__ Met cell_met_again(const double* p, int64_t cells) {
   double g[6], b[3];
 #pragma unroll
   for (int a = 0; a < 6; ++a) g[a] = p[cells * (GRB_GXX + a)];
