@@ -706,16 +706,14 @@ struct KScF {
   double D, iD, isD, q, r2, b2, rb2, bro, rBt;
   double ow, vmax;  // 1 - v_max^2 = 1 / (1 + r^2 / h0^2), v_max^2
 };
-// kRound: quotients and root correctly rounded, in the reference's order, for
-// the plain mode's iterates (W^2 / f', 10^5 in fast magnetised flows,
-// amplifies their rounding in the primitives).
-template <bool kRound>
+// Quotients and root are correctly rounded, in the reference's order, for the
+// plain mode's iterates (W^2 / f', 10^5 in fast magnetised flows, amplifies
+// their rounding in the primitives).
 GRB_HD void kscf(const DevEos& e, const Met& m, const double c[10], KScF& k) {
   k.D = c[0];
-  const double Df = k.D > 1e300 ? 1e300 : k.D;  // rcp_f and rsqrt_f of infinity are NaN
-  k.iD = kRound ? 1.0 / k.D : rcp_f(Df);
+  k.iD = 1.0 / k.D;
   k.q = c[4] * k.iD;
-  const double isD = kRound ? 1.0 / sqrt(k.D) : rsqrt_f(Df);
+  const double isD = 1.0 / sqrt(k.D);
   double r[3], Bt[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) { r[i] = c[1 + i] * k.iD; Bt[i] = c[7 + i] * isD; }
@@ -740,9 +738,8 @@ struct C2PLive {
   KScF k;
   double rup[3], s;
 };
-template <bool kRound>
 GRB_HD void c2p_live(const DevEos& e, const Met& m, const double c[10], C2PLive& L) {
-  kscf<kRound>(e, m, c, L.k);
+  kscf(e, m, c, L.k);
   mvs(m.gi, c + 1, L.rup);
 #pragma unroll
   for (int i = 0; i < 3; ++i) L.rup[i] *= L.k.iD;
@@ -852,66 +849,26 @@ struct EFn {
   }
 };
 
-// Root of an increasing f with f(0) < 0 by the secant method from x (first
-// step along slope 1, which f approaches for slow flows), kept inside the
-// bracket that the signs give (else its midpoint); past kSecantMax steps it
-// bisects.  Ends when the next step is below eps of x, or f below its own
-// rounding: 1 - v^2 carries an error of eps/2, which W^2 amplifies, and where
-// f' is small (1/100 in fast magnetised flows) a step repeats at that level
-// without shrinking; the slope is not taken from differences near it.  So the
-// primitives are as close to the sampled hybrid states' as Brent's (median
-// error 2.5e-13 in rho against 2.7e-13, backup solve 8.0e-14 against
-// 9.2e-14), in 3.1 evaluations on the blast wave's states where Brent from
-// [0, mu0] takes 6, 5.3 on the sampled states instead of 8.  f's members belong to the returned x.  NaN ends it.  clamp:
-// f is first visited at 0 and at x and f.clamp() called.
-constexpr int kSecantMax = 40;
-template <class Fn>
-GRB_HD double secant_root(Fn& f, double x, double top, bool clamp, int& iters, double& res) {
-  const double eps = 2.220446049250313e-16, x0 = x;
-  double lo = 0.0, hi = top, xp = 0.0, fp = 0.0, is = 1.0, ap = 1e300;
-  if (clamp) x = 0.0;
-  for (int it = clamp ? -2 : 0;; ++it) {
-    const double fx = f(x);
-    res = fx;
-    if (it < 0) {
-      f.clamp();
-      x = x0;
-      continue;
-    }
-    if (!(fx == fx)) break;
-    const double noise = (0.06 * eps) * x * (f.w * f.w);
-    const double df = fx - fp, af = fabs(fx);
-    if (it > 0 && fabs(df) > 280.0 * noise) is = (x - xp) * rcp_f(df);
-    const double d = fx * is, a = fabs(d);
-    if (it < kSecantMax ? (a <= eps * x || af <= noise || (af < 140.0 * noise && a >= 0.5 * ap))
-                        : (hi - lo <= eps * x || it > 3 * kSecantMax))
-      break;
-    if (fx > 0.0) hi = x; else lo = x;
-    ap = a;
-    xp = x;
-    fp = fx;
-    x -= d;
-    if (!(x > lo && x < hi) || it >= kSecantMax) x = 0.5 * (lo + hi);
-    ++iters;
-  }
-  return x;
-}
-
 // brent() from [0, top] with f evaluated at one place, and once more at the
-// root so that f's members belong to it.  For callers that want the plain
-// mode's iterates: the root then is the plain solve's own, to the last place
-// in most states, where two converged solvers differ by Brent's 1e-15.
+// root where that was not the last point, so that f's members belong to it.
+// The iterates are the plain mode's, so the root is the plain solve's own, to
+// the last place in most states, where two converged solvers differ by
+// Brent's 1e-15.  It ends only with f's two signs within the tolerance of each
+// other: in fast flows f at the bracket's top lies below its own rounding,
+// which W^2 amplifies, although the root is a factor away, so neither a small
+// |f| nor a small step tells a root.  (A secant iteration that stopped on
+// those took 3.1 evaluations instead of 6 on the blast wave's states and 4 to
+// 8 % less time a step, and returned the bracket's top for 7 in 1000 states of
+// an ideal gas of Gamma = 2 with eps to 1e4.)
 template <class Fn>
 GRB_HD double brent_root(Fn& f, double top, bool clamp, int& iters, double& res) {
   const double macheps = 2.220446049250313e-16;
   double sa = 0.0, sb = 0.0, fa = 0.0, fb = 0.0, c = 0.0, fc = 0.0, e = 0.0, d = 0.0;
   bool last = false;
   for (int it = -2;; ++it) {
-    const double fx = f(sb);
-    if (last) {
-      res = fx;
-      break;
-    }
+    const double x = sb, fx = f(x);
+    res = fx;
+    if (last) break;
     if (it < 0 && clamp) f.clamp();
     if (it == -2) {
       fa = fx;
@@ -934,6 +891,7 @@ GRB_HD double brent_root(Fn& f, double top, bool clamp, int& iters, double& res)
     const double tol = 2.0 * macheps * fabs(sb) + 1e-15;
     const double m = 0.5 * (c - sb);
     if (fabs(m) <= tol || fb == 0.0 || it >= kBrentMaxIter) {
+      if (it >= 0 && sb == x) break;  // (at the ends f.clamp() followed)
       last = true;
       continue;
     }
@@ -1033,9 +991,7 @@ GRB_HD void take_solution(const DevEos& e, const C2PLive& L, const Fn& f, double
 }
 
 // c2p_front in the tuned mode (plain bracket).
-// kBrent: the root by Brent's iteration from the plain bracket (the batch
-// entry points), else by secant_root (the stage passes).
-template <bool kBrent, bool kDry = false, class MetF>
+template <bool kDry = false, class MetF>
 GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const DevParams& P, double alp_bh_thresh,
                             C2PLive& L, MetF&& met) {
   C2PState F{};
@@ -1049,7 +1005,7 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
   pr[GRB_P_BX] = c[7]; pr[GRB_P_BY] = c[8]; pr[GRB_P_BZ] = c[9];
   F.lenient = m.alp < alp_bh_thresh;
   if (c[0] < 0) return F;  // c2p_back_f resets it to the atmosphere
-  kscf<kBrent>(e, m, c, k);
+  kscf(e, m, c, k);
   double ye = c[5] * k.iD;
   if (ye > e.yemax) { ye = e.yemax; o.err |= ERR_RESET_YE; }
   if (ye < 0.0) { ye = 0.0; o.err |= ERR_RESET_YE; }
@@ -1072,7 +1028,7 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
     if (st2 > qd * qd) {
       const double f = sqrt(qd * qd / st2);
       c[1] *= f; c[2] *= f; c[3] *= f;
-      kscf<kBrent>(e, m, c, k);
+      kscf(e, m, c, k);
       o.err |= ERR_RESET_STILDE;
       o.floored = true;
     }
@@ -1093,19 +1049,8 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
   f.e = &e;
   f.k = &k;
   F.mu0 = mu0_f(e, k);
-  double res, mu;
-  if (kBrent) {
-    mu = brent_root(f, F.mu0, false, o.iters, res);
-  } else {
-    // from 1/h of the fluid at rest for slow flows, else from the bracket's
-    // top, which fast flows come close to
-    double start = F.mu0;
-    if (k.r2 < e.h_min * e.h_min) {
-      const double eps0 = k.q - 0.5 * k.b2;
-      start = fmin(start, rcp_f(1.0 + (e.kind == GRB_EOS_IDEAL_GAS ? e.g : 1.0 + e.gthm1) * fmax(eps0, 0.0)));
-    }
-    mu = secant_root(f, start, e.ih0 * (1 + 1e-10), false, o.iters, res);
-  }
+  double res;
+  const double mu = brent_root(f, F.mu0, false, o.iters, res);
   o.mu = mu;
   // the signals of the full evaluation (kastaun_c2p.hh:245-290)
   if (f.vhigh) F.ret |= SIG_VEL_HIGH;
@@ -1136,7 +1081,7 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
 // c2p_backup in the tuned mode.  The reference's solve clamps the entropy to
 // its range at every density it visits and keeps it clamped: the range at
 // the bracket's two ends, its largest and smallest density, covers all.
-template <bool kBrent, class MetF>
+template <class MetF>
 GRB_HD void c2p_backup_f(C2PState& F, const C2PLive& L, double pr[13], const DevParams& P, MetF&& met) {
   const DevEos& e = P.eos;
   const bool ideal = e.kind == GRB_EOS_IDEAL_GAS;
@@ -1157,8 +1102,7 @@ GRB_HD void c2p_backup_f(C2PState& F, const C2PLive& L, double pr[13], const Dev
   const bool clamp = !(E0 * k.ow >= f.elo && E0 <= e.eps_max - ec0 && f.g <= 2.0);
   int it = 0;
   double res;
-  const double mu = kBrent ? brent_root(f, mu0, clamp, it, res)
-                           : secant_root(f, mu0, e.ih0 * (1 + 1e-10), clamp, it, res);
+  const double mu = brent_root(f, mu0, clamp, it, res);
   // (the clamps of eth would let a NaN entropy pass)
   if (s0 == s0 && fabs(res) <= P.tol && f.eps < e.eps_max) {
     uint32_t sig = 0;
@@ -1279,8 +1223,8 @@ GRB_HD C2POut c2p_f(double c[10], double pr[13], const Met& m, const DevParams& 
   C2PLive L;
   const bool ex = excised(P, m.alp, r_sph);
   const double sqrtg = m.sqrtg;
-  C2PState F = c2p_front_f<false>(c, pr, m, P, alp_bh_thresh, L, met);
-  if (F.backup) c2p_backup_f<false>(F, L, pr, P, met);
+  C2PState F = c2p_front_f(c, pr, m, P, alp_bh_thresh, L, met);
+  if (F.backup) c2p_backup_f(F, L, pr, P, met);
   c2p_back_f<kAllCons>(F, c, pr, sqrtg, P, ex, met);
   return F.o;
 }
@@ -1288,7 +1232,7 @@ template <class MetF>
 GRB_HD bool c2p_floored_f(double c[10], double pr[13], const Met& m, const DevParams& P, double r_sph, MetF&& met) {
   C2PLive L;
   const bool ex = excised(P, m.alp, r_sph);
-  C2PState F = c2p_front_f<false, true>(c, pr, m, P, 1e30, L, met);
+  C2PState F = c2p_front_f<true>(c, pr, m, P, 1e30, L, met);
   if (!F.done) c2p_back_f<true, true>(F, c, pr, 0.0, P, ex, met);
   return F.o.floored;
 }

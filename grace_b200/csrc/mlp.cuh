@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kC2PThreads, kDefer && !kLearned ? 4 : 1) k_c2
   C2PLive L;
   if (active) {
     F = kLearned ? c2p_front<true>(c, pr, m, P, false, P.alp_bh_thresh, gs)
-                 : c2p_front_f<true>(c, pr, m, P, P.alp_bh_thresh, L, met);
+                 : c2p_front_f(c, pr, m, P, P.alp_bh_thresh, L, met);
   }
   const bool later = kDefer && active && !F.done && F.backup;
   // one slot per deferred lane, one atomic per warp
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kC2PThreads, kDefer && !kLearned ? 4 : 1) k_c2
     d.t = t;
     return;
   }
-  if (!kDefer && F.backup) c2p_backup_f<true>(F, L, pr, P, met);
+  if (!kDefer && F.backup) c2p_backup_f(F, L, pr, P, met);
   if (!F.done) c2p_back_f(F, c, pr, m.sqrtg, P, excised(P, m.alp, 0.0), met);
   if (F.o.fatal) atomicOr(flags, F.o.fatal);
   pr[GRB_P_CS2] = 0.0;
@@ -538,8 +538,8 @@ __global__ void __launch_bounds__(kC2PThreads, 4) k_c2p_batch_backup(DevParams P
     const Met m = batch_metric<true>(metric, n, t);
     const auto met = [&] { return batch_metric_again(metric, n, t); };
     C2PLive L;
-    c2p_live<true>(P.eos, m, c, L);
-    c2p_backup_f<true>(F, L, pr, P, met);
+    c2p_live(P.eos, m, c, L);
+    c2p_backup_f(F, L, pr, P, met);
     c2p_back_f(F, c, pr, m.sqrtg, P, excised(P, m.alp, 0.0), met);
     if (F.o.fatal) atomicOr(flags, F.o.fatal);
     pr[GRB_P_CS2] = 0.0;

@@ -1203,7 +1203,7 @@ __global__ void __launch_bounds__(128, MINB) k_aux_front(DevParams P, Geo G, Box
     m = aux_load<true>(G, i, j, k, q, st, bx, by, bz, aux, idx, true, c);
     s0 = st + cvar(G, i, j, k, 0, GRB_N_EVOL_VARS, q);
     ex = excised(P, m.alp, cell_r(G, coords, idx + 3 * q, i, j, k, q));
-    F = c2p_front_f<false>(c, pr, m, P, P.alp_bh_thresh, L, met);
+    F = c2p_front_f(c, pr, m, P, P.alp_bh_thresh, L, met);
   }
   const bool later = active && F.backup;
   const unsigned mask = __ballot_sync(0xffffffffu, later);
@@ -1222,7 +1222,7 @@ __global__ void __launch_bounds__(128, MINB) k_aux_front(DevParams P, Geo G, Box
       d.F = F;
       d.i = i; d.j = j; d.k = k; d.q = q;
     } else {
-      if (F.backup) c2p_backup_f<false>(F, L, pr, P, met);
+      if (F.backup) c2p_backup_f(F, L, pr, P, met);
       c2p_back_f<false>(F, c, pr, m.sqrtg, P, ex, met);
       dtc = aux_finish<kDt, true>(P, G, i, j, k, q, st, bx, by, bz, aux, m, c, pr, F.o, B, dta);
     }
@@ -1254,8 +1254,8 @@ __global__ void __launch_bounds__(128, MINB) k_aux_backup(DevParams P, Geo G, do
     for (int v = 0; v < 13; ++v) pr[v] = d.pr[v];
     C2PState F = d.F;
     C2PLive L;
-    c2p_live<false>(P.eos, m, c, L);
-    c2p_backup_f<false>(F, L, pr, P, met);
+    c2p_live(P.eos, m, c, L);
+    c2p_backup_f(F, L, pr, P, met);
     c2p_back_f<false>(F, c, pr, m.sqrtg, P, excised(P, m.alp, cell_r(G, coords, idx + 3 * q, i, j, k, q)), met);
     dtc = fmin(dtc, aux_finish<kDt, true>(P, G, i, j, k, q, st, bx, by, bz, aux, m, c, pr, F.o, B, dta));
   }
