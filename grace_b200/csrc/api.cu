@@ -320,18 +320,15 @@ bool launch_flux_tma(cudaStream_t s, const DevParams& P, const Geo& G, const Box
 // 64 blocks of 16^3 take 1500 us against 1358.
 constexpr int64_t kFluxMergeTiles = 148 * 4;
 template <int MINB, int NT>
-bool launch_flux_tma3(cudaStream_t s, const DevParams& P, const Geo& G, const double* st, const double* aux,
-                      const double* const bf[3], const StageBufs& B) {
+bool launch_flux_tma3(grb_handle* h, cudaStream_t s, const DevParams& P, const Geo& G, const double* st,
+                      const double* aux, const double* const bf[3], const StageBufs& B) {
   FluxTma3 A;
   size_t smem = 0;
   int64_t tiles = 0;
+  if (G.nq > 65535) return false;
   for (int d = 0; d < 3; ++d) {
-    const Box b = face_box(G, P.emf, d, G.nq);
-    A.T[d] = flux_tile(d, G, b, NT);
-    if (A.T[d].R < 1 || b.nq > 65535) return false;
-    if (!make_tmap(&A.aux[d], aux, G, GRB_N_AUX_VARS, b.nq, A.T[d]) ||
-        !make_tmap(&A.met[d], st, G, GRB_N_EVOL_VARS, b.nq, A.T[d]))
-      return false;
+    A.T[d] = flux_tile(d, G, face_box(G, P.emf, d, G.nq), NT);
+    if (A.T[d].R < 1) return false;
     A.bf[d] = bf[d];
     smem = std::max(smem, flux_tile_smem(G, A.T[d]));
     const int nrow = d == 2 ? A.T[d].n[2] : A.T[d].n[1], nother = d == 2 ? A.T[d].n[1] : A.T[d].n[2];
@@ -339,7 +336,11 @@ bool launch_flux_tma3(cudaStream_t s, const DevParams& P, const Geo& G, const do
     A.first[d] = (int)tiles;
     tiles += (int64_t)A.ntx[d] * nother;
   }
-  if (tiles * G.nq > kFluxMergeTiles || tiles > 0x7fffffff) return false;
+  if (tiles * G.nq > kFluxMergeTiles) return false;
+  for (int d = 0; d < 3; ++d)
+    if (!make_tmap(&A.aux[d], aux, G, GRB_N_AUX_VARS, G.nq, A.T[d]) ||
+        !make_tmap(&A.met[d], st, G, GRB_N_EVOL_VARS, G.nq, A.T[d]))
+      return false;
   static size_t attr[kMaxDevices] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
@@ -349,6 +350,7 @@ bool launch_flux_tma3(cudaStream_t s, const DevParams& P, const Geo& G, const do
       return false;
     attr[dev] = smem;
   }
+  KScope ks(h, s, GRB_KIND_FLUX);  // only now: a scope around no launch would count as one
   k_flux_tma3<MINB, NT><<<dim3((unsigned)tiles, 1, (unsigned)G.nq), NT, smem, s>>>(P, G, A, B);
   return true;
 }
@@ -761,9 +763,8 @@ int stage_tuned(grb_handle* h, const Geo& G, const grb_grid* g, double dt, doubl
   const double* bf[3] = {old->bx, old->by, old->bz};
   bool merged = false;
   if (h->var_flux == 1 || h->var_flux == 2) {
-    KScope ks(h, s, GRB_KIND_FLUX);
-    merged = h->var_flux == 1 ? launch_flux_tma3<4, 128>(s, P, G, old->state, aux, bf, B)
-                              : launch_flux_tma3<2, 256>(s, P, G, old->state, aux, bf, B);
+    merged = h->var_flux == 1 ? launch_flux_tma3<4, 128>(h, s, P, G, old->state, aux, bf, B)
+                              : launch_flux_tma3<2, 256>(h, s, P, G, old->state, aux, bf, B);
     launches += merged;
   }
   for (int dir = 0; dir < 3 && !merged; ++dir) {

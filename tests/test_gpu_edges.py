@@ -52,6 +52,28 @@ def test_flux_tiles_match_oracle(flux, nb, n, recon):
     assert g.status().device_flags == 0
 
 
+# one launch up to a wave of tiles, else one a direction; every timed scope is a launch
+@pytest.mark.parametrize("nb,launches", [((3, 3, 2), 1), ((5, 2, 2), 3)])
+@pytest.mark.parametrize("flux", [0, 1, 2])
+def test_flux_launches_are_counted_once(flux, nb, launches):
+    su, (st, bx, by, bz, aux) = workloads.blast(nb=nb, n=(8, 8, 8))
+    g = GRMHDEquationsSystem(params.blast())
+    g.reserve(Blocks(*su.n, su.ngz, su.nq, su.idx(), device="cuda:0"))
+    g.set_mode(abi.MODE_TUNED)
+    g.set_tuning(flux=flux)
+    old, a = Fields(dev(st), dev(bx), dev(by), dev(bz)), dev(aux)
+    new = old.clone()
+    g.compute_auxiliary_quantities(old, a)
+    g.set_kernel_timing(True)
+    before = g.status().launches
+    g.advance_substep(0.0, 1e-3, 1.0, new, old, a)
+    count = {k: c for k, (_, c) in g.kernel_times().items()}
+    assert count["flux"] == (launches if flux else 3)
+    # flux, EMF, flag, the three FOFC passes (one scope), update, CT
+    assert g.status().launches - before == count["flux"] + 7
+    assert sum(count.values()) == count["flux"] + 5
+
+
 # 24 is the largest interior whose contractions fit shared memory
 @pytest.mark.parametrize("n", [6, 10, 22, 24, 26])
 def test_fmr_restriction_sizes_match_oracle_bitwise(n):
