@@ -10,9 +10,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <random>
 #include <tuple>
 #include <utility>
@@ -287,6 +289,25 @@ bool make_tmap(CUtensorMap* tm, const double* base, const Geo& G, int nv, int64_
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+// Allows `kernel` that much dynamic shared memory on the current device.  The
+// attribute is per kernel and device, and is only ever raised, under a lock:
+// host threads with handles of their own share it, and a smaller value set
+// late would fail another thread's launch.
+template <auto kernel>
+bool allow_smem(size_t bytes) {
+  static std::atomic<size_t> got[kMaxDevices];
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+  if (bytes <= got[dev].load(std::memory_order_acquire)) return true;
+  const std::lock_guard<std::mutex> lock(mu);
+  if (bytes <= got[dev].load(std::memory_order_relaxed)) return true;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+    return false;
+  got[dev].store(bytes, std::memory_order_release);
+  return true;
+}
+
 template <int dir, int MINB, int NT = 128>
 bool launch_flux_tma(cudaStream_t s, const DevParams& P, const Geo& G, const Box& b, const double* st,
                      const double* aux, const double* bf, const StageBufs& B) {
@@ -296,16 +317,7 @@ bool launch_flux_tma(cudaStream_t s, const DevParams& P, const Geo& G, const Box
   if (!make_tmap(&ta, aux, G, GRB_N_AUX_VARS, b.nq, T) || !make_tmap(&tm, st, G, GRB_N_EVOL_VARS, b.nq, T))
     return false;
   const size_t smem = flux_tile_smem(G, T);
-  // the attribute is per device: remember what each device ordinal got
-  static size_t attr[kMaxDevices] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
-  if (smem > attr[dev]) {
-    if (cudaFuncSetAttribute(k_flux_tma<dir, MINB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return false;
-    attr[dev] = smem;
-  }
+  if (!allow_smem<k_flux_tma<dir, MINB, NT>>(smem)) return false;
   const int nrow = dir == 2 ? T.n[2] : T.n[1];
   const int nother = dir == 2 ? T.n[1] : T.n[2];
   const dim3 grid((unsigned)((nrow + T.R - 1) / T.R), (unsigned)nother, (unsigned)b.nq);
@@ -341,15 +353,7 @@ bool launch_flux_tma3(grb_handle* h, cudaStream_t s, const DevParams& P, const G
     if (!make_tmap(&A.aux[d], aux, G, GRB_N_AUX_VARS, G.nq, A.T[d]) ||
         !make_tmap(&A.met[d], st, G, GRB_N_EVOL_VARS, G.nq, A.T[d]))
       return false;
-  static size_t attr[kMaxDevices] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
-  if (smem > attr[dev]) {
-    if (cudaFuncSetAttribute(k_flux_tma3<MINB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return false;
-    attr[dev] = smem;
-  }
+  if (!allow_smem<k_flux_tma3<MINB, NT>>(smem)) return false;
   KScope ks(h, s, GRB_KIND_FLUX);  // only now: a scope around no launch would count as one
   k_flux_tma3<MINB, NT><<<dim3((unsigned)tiles, 1, (unsigned)G.nq), NT, smem, s>>>(P, G, A, B);
   return true;
@@ -388,17 +392,10 @@ bool launch_flux_tma_queue(cudaStream_t s, const DevParams& P, const Geo& G, con
   if (!make_tmap(&ta, aux, G, GRB_N_AUX_VARS, b.nq, T) || !make_tmap(&tm, st, G, GRB_N_EVOL_VARS, b.nq, T))
     return false;
   const size_t smem = flux_tile_smem(G, T);
-  static size_t attr[kMaxDevices] = {};
   static int occ_for[kMaxDevices] = {};
   static size_t occ_smem[kMaxDevices] = {};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
-  if (smem > attr[dev]) {
-    if (cudaFuncSetAttribute(k_flux_tma_queue<dir, MINB, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return false;
-    attr[dev] = smem;
-  }
+  if (!allow_smem<k_flux_tma_queue<dir, MINB, NT>>(smem) || cudaGetDevice(&dev) != cudaSuccess) return false;
   if (occ_smem[dev] != smem) {
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_flux_tma_queue<dir, MINB, NT>, NT, smem) !=
@@ -1448,34 +1445,12 @@ int grb_mlp_eval(grb_handle* h, int64_t n, const float* params, const float* fea
 namespace {
 constexpr int kKeepParts = 1024;  // 39 MB
 int grad_setup(grb_handle* h) {
-  static bool done = false;
-  if (!done) {
-    CK(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpGradSmem)));
-    done = true;
-  }
-  return GRB_OK;
+  return allow_smem<k_mlp_grad>(sizeof(MlpGradSmem)) ? GRB_OK : fail(h, GRB_ERR_CUDA);
 }
 }  // namespace
 
-// Shared memory a CTA of the FMR kernels may take (two per SM), and the
-// attribute that allows it, per kernel and device.
+// Shared memory a CTA of the FMR kernels may take (two per SM).
 constexpr size_t kFmrSmem = 100 << 10;
-template <class... A>
-static bool fmr_smem(void (*kernel)(A...)) {
-  static void* done[kMaxDevices][8] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
-  for (void*& k : done[dev]) {
-    if (k == reinterpret_cast<void*>(kernel)) return true;
-    if (!k) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFmrSmem) != cudaSuccess)
-        return false;
-      k = reinterpret_cast<void*>(kernel);
-      return true;
-    }
-  }
-  return false;
-}
 
 // FMR prolongation launches of one element kind (grb_prolong_to_ghosts).
 template <int kKind>
@@ -1500,7 +1475,7 @@ static void launch_prolong(const Geo& G, const int ext[3], const grb_fields* fin
     smem = std::max(smem, sizeof(double) * kV * 2 * r[0] * (r[2] + 4) * (size_t)(r[1] + 4 + 2 * r[1]));
   }
   const int groups = (V[1].n + kV - 1) / kV;
-  if (V[1].n && smem <= kFmrSmem && groups * nelems <= 0x7fffffff && fmr_smem(k_prolong_lag<kKind, kV>)) {
+  if (V[1].n && smem <= kFmrSmem && groups * nelems <= 0x7fffffff && allow_smem<k_prolong_lag<kKind, kV>>(kFmrSmem)) {
     ProlongDivs D;
     const int ext6[6] = {G.nx / 2, G.g / 2, G.nx / 2 + 4, G.g / 2 + 4, G.nx, G.g};
     for (int k = 0; k < 6; ++k) D.d[k] = make_fastdiv((uint32_t)ext6[k]);
@@ -2063,7 +2038,7 @@ int grb_restrict_to_coarse(grb_handle* h, const grb_grid* g, const grb_fields* f
       // below 6 cells along y or z the stencils reach ghost cells, which the
       // staged interior does not hold
       if (G.nx <= 256 && G.ny >= 6 && G.nz >= 6 && smem <= kFmrSmem && (int64_t)nl * nquads <= 0x7fffffff &&
-          fmr_smem(k_restrict_lag)) {
+          allow_smem<k_restrict_lag>(kFmrSmem)) {
         k_restrict_lag<<<(unsigned)(nl * nquads), 128, smem, s>>>(
             G, V, make_fastdiv((uint32_t)nl), fine->state, cbuf->state, src_q, dst_q, child_id);
       } else if (G.nz < 6) {

@@ -175,6 +175,58 @@ def test_c2p_odd_conservatives_match_oracle():
         np.testing.assert_array_equal(np.isfinite(got[0, v]), np.isfinite(aux_o[0, v]))
 
 
+def test_handles_of_several_threads():
+    """Four host threads, each with a handle and a stream of its own, whose
+    tiles want different amounts of shared memory: a substep in both tile
+    sizes and an FMR restriction and prolongation, ten times over, bit for bit
+    what one thread gets."""
+    from concurrent.futures import ThreadPoolExecutor
+    sizes = [(28, 8, 10), (58, 8, 8), (120, 8, 8), (8, 8, 8)]
+    rng = np.random.default_rng(91)
+
+    def case(k):
+        su, f = workloads.blast(nb=(1, 1, 1), n=sizes[k])
+        n = (6, 10, 22, 24)[k]
+        return su, f, n, rng.standard_normal((8, abi.N_EVOL_VARS) + (n + 2 * G,) * 3)
+
+    cases = [case(k) for k in range(4)]
+
+    def work(k):
+        torch.cuda.set_device(0)
+        su, (st, bx, by, bz, aux), n, fine = cases[k]
+        out = []
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for flux in (1, 2):
+                g = GRMHDEquationsSystem(params.blast())
+                g.reserve(Blocks(*su.n, su.ngz, su.nq, su.idx(), device="cuda:0"))
+                g.set_mode(abi.MODE_TUNED)
+                g.set_tuning(flux=flux)
+                old, a = Fields(dev(st), dev(bx), dev(by), dev(bz)), dev(aux)
+                new = old.clone()
+                g.compute_auxiliary_quantities(old, a)
+                g.advance_substep(0.0, 1e-3, 1.0, new, old, a)
+                out += [new.state, new.bx]
+            q = np.arange(8, dtype=np.int64)
+            g = GRMHDEquationsSystem(params.blast())
+            g.reserve(Blocks(n, n, n, G, 8, np.ones((8, 3)), device="cuda:0"))
+            F = Fields(dev(fine), None, None, None)
+            C = Fields(torch.zeros_like(F.state), None, None, None)
+            g.restrict_to_coarse(F, C, dev(q), dev(q), dev(q.astype(np.uint8)), [], [1, 7, 22], faces=False)
+            g.prolong_to_ghosts(F, C, 0, dev(q[:6]), dev(q[:6]), dev(q[:6].astype(np.uint8)), None, [], [1, 7],
+                                faces=False)
+            out += [C.state, F.state]
+            torch.cuda.current_stream().synchronize()
+        return [x.cpu().numpy() for x in out]
+
+    with ThreadPoolExecutor(4) as pool:  # before the one-thread run: the limits are still to be raised
+        runs = [list(pool.map(work, range(4))) for _ in range(10)]
+    want = [work(k) for k in range(4)]
+    for run in runs:
+        for got, ref in zip(run, want):
+            for x, y in zip(got, ref):
+                np.testing.assert_array_equal(x, y)
+
+
 @pytest.mark.parametrize("shift", [0, 1])
 @pytest.mark.parametrize("n", [(5, 6, 7), (16, 4, 5)])
 def test_linop_unaligned_arrays(n, shift):
