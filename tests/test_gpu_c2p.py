@@ -154,3 +154,26 @@ def test_c2p_edge_cases():
     assert err_g[0] & (1 << 20) and err_g[3] & (1 << 20)  # C2P_ATMO_RESET
     rel = np.abs(pr_g[abi.P_RHO] - pr_o[abi.P_RHO]) / pr_o[abi.P_RHO]
     assert np.all(rel < prim_tol(pr_o))
+
+
+@pytest.mark.parametrize("n", [3000, 45000])
+def test_tuned_c2p_with_negative_cold_energies_matches_oracle(n):
+    """A cold table whose energies are negative (an offset of -0.05, as binding
+    energies give): states with eps between that and 0 are inside the equation
+    of state's range and keep their tau, in place and deferred batches."""
+    P = params.c2p_bench()
+    P.eos.pw_eps[0] = -0.05
+    rng = np.random.default_rng(23)
+    rho, eth = 10 ** rng.uniform(-10, -4, n), 10 ** rng.uniform(-6, -1, n)
+    eps = -0.05 + 100.0 * rho + eth
+    z = rng.standard_normal((3, n)) * 10 ** rng.uniform(-3, 0, n)
+    B = rng.standard_normal((3, n)) * np.sqrt(rho) * 10 ** rng.uniform(-3, 0, n)
+    s = np.log(eth * rho ** -0.8) / 0.8
+    cons = np.zeros((10, n))
+    cons[:7] = workloads.flat_prims_to_cons(rho, 100.0 * rho ** 2 + 0.8 * rho * eth, eps, z, B, s)
+    cons[7:] = B
+    pr_g, _, err_g, pr_o, _, err_o = _compare(P, cons, mode=abi.MODE_TUNED)
+    assert np.mean(eps < 0) > 0.5
+    same = err_g == err_o
+    assert same.mean() > 0.999
+    assert np.all(state_residual(pr_g[:, same], pr_o[:, same]) < prim_tol(pr_o)[same])
