@@ -824,17 +824,13 @@ struct EFn {
     w = rsqrt_f(om);
     iw = om * w;
     rho = k->D * iw;
-    double lr = 0.5 * log(om), pr = 0.0, ec = 0.0;
-    if (e->kind != GRB_EOS_IDEAL_GAS) {
-      double irho = w * k->iD;
-      double r = rho;
-      if (rho > e->rhomax || rho < e->rhomin) {
-        r = clamp_f(rho, e->rhomin, e->rhomax);
-        irho = rcp_f(r);
-        lr = log(r * k->iD);
-      }
-      pw_cold_f(*e, r, irho, pr, ec);
+    double lr = 0.5 * log(om), pr = 0.0, ec = 0.0, r = rho, irho = w * k->iD;
+    if (rho > e->rhomax || rho < e->rhomin) {
+      r = clamp_f(rho, e->rhomin, e->rhomax);
+      irho = rcp_f(r);
+      lr = log(r * k->iD);
     }
+    if (e->kind != GRB_EOS_IDEAL_GAS) pw_cold_f(*e, r, irho, pr, ec);
     raw = exp(g * (sl + lr));
     hi = e->eps_max - ec;
     eth = raw > elo ? raw : elo;

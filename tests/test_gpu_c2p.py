@@ -177,3 +177,21 @@ def test_tuned_c2p_with_negative_cold_energies_matches_oracle(n):
     same = err_g == err_o
     assert same.mean() > 0.999
     assert np.all(state_residual(pr_g[:, same], pr_o[:, same]) < prim_tol(pr_o)[same])
+
+
+@pytest.mark.parametrize("n", [500, 40000])
+def test_tuned_c2p_backup_beyond_the_density_range_matches_oracle(n):
+    """Ideal gas at D above the largest density (1e100), entropies that give
+    a moderate eps there: the Kastaun solve is distrusted, and the backup takes
+    the entropy at the clamped density."""
+    P = params.ideal_gas(5.0 / 3.0)
+    rng = np.random.default_rng(29)
+    D, eps = 10 ** rng.uniform(100.1, 101, n), 10 ** rng.uniform(-2, 1, n)
+    cons = np.zeros((10, n))
+    cons[0], cons[4] = D, D * eps
+    cons[6] = D * (np.log(eps) * 1.5 - 100.0 * np.log(10.0))
+    pr_g, _, err_g, pr_o, _, err_o = _compare(P, cons, mode=abi.MODE_TUNED)
+    np.testing.assert_array_equal(err_g, err_o)
+    for v in (abi.P_RHO, abi.P_EPS, abi.P_PRESS, abi.P_TEMP):
+        # eps is exp of a sum of numbers of up to 345, rounded in either order
+        np.testing.assert_allclose(pr_g[v], pr_o[v], rtol=8 * 345 * 2.0 ** -52, err_msg=str(v))
