@@ -82,10 +82,12 @@ struct DevParams {
 // and 1/sqrt(x) = y (1 + e/2 + 3 e^2/8) + O(e^3) (the binomial series), so
 // the truncation (|e| < 2^-18) is below the rounding of the last operation.
 // 3 to 5 FP64 instructions and no branch, where the correctly rounded forms
-// take two to three times as many; the results are within 1 to 2 units in
-// the last place, as the products of paired quotients that they replace were.
-// For finite x of normal magnitude (rcp_f: either sign, 1/x normal too;
-// rsqrt_f: x > 0; sqrt_f: x >= 0, 0 below 1e-290).
+// take two to three times as many; rcp_f is within 1, the roots within 2 units
+// in the last place, as the products of paired quotients that they replace
+// were.  For finite x of normal magnitude (rcp_f: either sign, 1/x normal too;
+// rsqrt_f: x > 0; sqrt_f: x >= 0).  Beyond: NaN at infinity and NaN, for rcp_f
+// and rsqrt_f also at 0; rcp_f of a subnormal or with a subnormal result is
+// not a reciprocal; sqrt_f gives 0 at 0 and less than 1e-145 below 1e-290.
 GRB_HD double rcp_f(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
