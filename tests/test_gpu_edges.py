@@ -267,3 +267,25 @@ def test_mlp_gradient_sizes_match_oracle(n):
     tol = 3 * 2.0 ** -8
     assert abs(loss - loss_o) <= tol * loss_o
     assert np.linalg.norm(got.cpu().numpy() - want) <= tol * np.linalg.norm(want)
+
+
+# 2, 10, 16 and 1025 tiles (the last: an own buffer); the sums take every eighth row
+@pytest.mark.parametrize("n,tiles", [(65, (0, 1)), (581, (0, 7, 8, 9)), (1024, (0, 7, 8, 15)),
+                                     (65600, (0, 7, 8, 511, 1023, 1024))])
+def test_mlp_gradient_counts_every_tile_once(n, tiles):
+    """Targets on the network's own outputs except in one tile of 64 samples,
+    which then is the whole gradient and loss: left out or taken twice, either
+    is off by its full size."""
+    P = random_params(9)
+    _, f, _ = feats_targets(n, 48)
+    s = GRMHDEquationsSystem(params.c2p_bench())
+    fit = s.mlp_eval(dev(f), dev(P)).cpu().numpy()
+    for k in tiles:
+        t, at = fit.copy(), slice(64 * k, min(64 * (k + 1), n))
+        t[at] *= 1.5
+        got, loss = s.mlp_grad(dev(P), dev(f), dev(t))
+        loss_o, want = _oracle.mlp_loss_grad(P, np.ascontiguousarray(f[:, at]), t[at], emulate=True)
+        share = (at.stop - at.start) / n
+        tol = 3 * 2.0 ** -8  # as above
+        assert abs(loss / share - loss_o) <= tol * loss_o, k
+        assert np.linalg.norm(got.cpu().numpy() / share - want) <= tol * np.linalg.norm(want), k
