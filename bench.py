@@ -652,12 +652,12 @@ def ours(args, rank, world, local_rank):
             leg["peak_source"] = peak_src
     top = max(kt.items(), key=lambda kv: kv[1][0])
     name, (kms, kcnt) = top
-    # faces one flux launch (one direction) computes: the reference's full
-    # transverse ghost range in the plain form, only the faces the stage
-    # reads in the tuned form (GS: n+2 transverse, UCT: n+6)
-    tr = (n + 8) if args.mode != "tuned" else ((n + 2) if P.emf == abi.EMF_GS else (n + 6))
+    # faces one flux launch computes: those the stage reads of one direction
+    # (n+2 transverse for GS, n+6 for UCT; both modes), of all three where a
+    # small grid's stage takes one launch (the timed launches tell)
+    tr = (n + 2) if P.emf == abi.EMF_GS else (n + 6)
     items = {
-        "flux": nq * (n + 3) * tr ** 2,
+        "flux": nq * (n + 3) * tr ** 2 * 9 * args.steps // max(kt["flux"][1], 1),
         "aux": nq * (n + 8) ** 3,
         "update": nq * n ** 3,
     }
