@@ -1006,14 +1006,17 @@ GRB_HD C2PState c2p_front_f(double c[10], double pr[13], const Met& m, const Dev
   if (ye > e.yemax) { ye = e.yemax; o.err |= ERR_RESET_YE; }
   if (ye < 0.0) { ye = 0.0; o.err |= ERR_RESET_YE; }
   pr[GRB_P_YE] = ye;
-  // limit_conservatives (c2p.cpp:117-157); the least eps, negative only where
-  // the cold table's offsets are, is formed for the states below 0
-  const double B2 = sqs(m.g, c + 7), eps0 = k.q - 0.5 * B2 * k.iD;
-  if (eps0 < 0.0) {
+  // limit_conservatives (c2p.cpp:117-157): tau below min(0, least eps).  The
+  // least eps, negative only where the cold table's offsets are, is formed for
+  // the states below 0 alone, and compared through the tau it gives (a value
+  // less live: this kernel's registers are full).
+  const double B2 = sqs(m.g, c + 7);
+  if (k.q - 0.5 * B2 * k.iD < 0.0) {
     double lo, hi;
     eos_eps_range(e, lo, hi, c[0]);
-    if (eps0 < fmin(0.0, lo)) {
-      c[4] = lo * c[0] + 0.5 * B2;
+    const double tau = lo * c[0] + 0.5 * B2;
+    if (lo >= 0.0 || c[4] < tau) {
+      c[4] = tau;
       k.q = c[4] * k.iD;
       o.err |= ERR_RESET_TAU;
       o.floored = true;
