@@ -976,6 +976,9 @@ int grb_reserve(grb_handle* h, const grb_grid* g) {
   if (h->B.ecenter) CK(cudaMemset(h->B.ecenter, 0, sizeof(double) * nc * 3));
   if (h->B.vbar) CK(cudaMemset(h->B.vbar, 0, sizeof(double) * nf * 4 * 3));
   CK(cudaDeviceSynchronize());
+  // valid for whoever runs the flag kernel; a substep on fewer blocks moves the
+  // edge tags down behind its face tags, to clear both at once
+  h->B.etag = h->B.ftag + nf * 3;
   h->geo = G;
   h->cap_f = nf;
   h->cap_c = nc;

@@ -287,3 +287,34 @@ def test_deferred_backup_aux_pass_matches_oracle(aux):
     backup = (ga[:, abi.C2P_ERR][sel].astype(np.uint64) >> 19) & 1
     assert backup.mean() > 0.5
     assert g.status().device_flags == 0
+
+
+def test_autotune_on_cells_that_fofc_flags():
+    """Excised cells (lapse below alp_ex) are flagged whatever the fluxes, also
+    by the flag kernel's timing runs; the autotuner leaves nothing behind that a
+    substep sees."""
+    P = params.blast()
+    su, (st, bx, by, bz, aux) = workloads.blast(nb=(2, 2, 2), n=(8, 8, 8))
+    st = st.copy()
+    st[:, abi.ALP, 6:9, 7:10, 5:8] = 0.5 * P.alp_ex
+    T = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to("cuda:0")
+    out = []
+    for tuned in (False, True):
+        g = GRMHDEquationsSystem(P)
+        g.reserve(Blocks(*su.n, su.ngz, su.nq, su.idx(), device="cuda:0"))
+        g.set_mode(abi.MODE_TUNED)
+        old, a = Fields(T(st), T(bx), T(by), T(bz)), T(aux)
+        new = old.clone()
+        g.compute_auxiliary_quantities(old, a)
+        if tuned:
+            g.autotune(new, old, a)
+            g.set_tuning(1, 1, 1, 1)
+        else:
+            g.set_tuning(1, 1, 1, 1)
+        g.advance_substep(0.0, 1e-3, 1.0, new, old, a)
+        s = g.status()
+        assert s.fofc_faces > 0 and s.device_flags == 0
+        out.append((s.fofc_faces, s.fofc_edges, new.state.cpu().numpy(), new.bx.cpu().numpy()))
+    assert out[0][:2] == out[1][:2]
+    for x, y in zip(out[0][2:], out[1][2:]):
+        np.testing.assert_array_equal(x, y)
