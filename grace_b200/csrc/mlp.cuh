@@ -423,17 +423,19 @@ struct C2PDeferred {
   int64_t t;
 };
 
-//
 // 4 CTAs per SM (128 registers, at most 140 bytes of spills in the backup):
 // at 3, the uncapped 136 and 168 registers, 2 M states took 1008 us against
 // 873; the dependent chains of the solves want warps more than registers.
+// With the network 3 (168 registers): left free it takes 178 and holds 2, and
+// 2^24 states go at 5.4e8 a second instead of 5.8e8, the TOV star's cells at
+// 1.26e9 instead of 1.41e9.
 // kDefer false: a batch of at most kC2PDirect states (two warps a scheduler)
 // runs the backups in place: with the GPU mostly empty there is nothing to
 // compact, and the second launch, its wait for the first and the cleared
 // count cost more than divergent warps.
 constexpr int64_t kC2PDirect = 148 * 2 * kC2PThreads;
 template <bool kLearned, bool kDefer = true>
-__global__ void __launch_bounds__(kC2PThreads, kDefer && !kLearned ? 4 : 1) k_c2p_batch_front(DevParams P, int64_t n,
+__global__ void __launch_bounds__(kC2PThreads, kLearned ? 3 : kDefer ? 4 : 1) k_c2p_batch_front(DevParams P, int64_t n,
                                                                 const double* __restrict__ cons,
                                                                 const double* __restrict__ metric,
                                                                 double* __restrict__ prims,
