@@ -47,13 +47,13 @@ ALGO_BYTES = {
 # cudaProfilerStart/Stop, every launch, cold L2 per kernel), scaled to a full
 # launch by the items it computes:
 #   the TMA-staged flux kernel (mean of the three directions), per face:
-FLUX_DRAM_BYTES_PER_FACE = 310.2      # dram__bytes_read.sum + dram__bytes_write.sum
+FLUX_DRAM_BYTES_PER_FACE = 311.3      # dram__bytes_read.sum + dram__bytes_write.sum
 FLUX_FP64_FLOP_PER_FACE = 1568.6      # dadd + dmul + 2 dfma (thread instructions)
 FLUX_FP64_INST_PER_FACE = 1110.9      # dadd + dmul + dfma
 #   the whole RK3 step (42 launches), per zone-update:
-STEP_DRAM_BYTES_PER_ZU = 4651.6
-STEP_FP64_FLOP_PER_ZU = 10140.6
-STEP_FP64_INST_PER_ZU = 7180.8
+STEP_DRAM_BYTES_PER_ZU = 4805.2
+STEP_FP64_FLOP_PER_ZU = 11474.3
+STEP_FP64_INST_PER_ZU = 8054.3
 # algorithmic FP64 bytes per zone-update: 66 doubles on RK3 stage 1, 76 on
 # stages 2 and 3 (they also read the u^n combination), 581 B averaged
 ALGO_BYTES_PER_ZU = 581.0
