@@ -410,7 +410,7 @@ int grb_mlp_grad(grb_handle* h, int64_t n, const float* params,
  * variables.
  * GRB_MODE_TUNED: the same faces from shared-memory tiles, one reciprocal per
  * face for the HLL fluxes and per WENO-Z state, the register-cap variant
- * picked by grb_autotune, fewer divisions and evaluations in the c2p.
+ * picked by grb_autotune, fewer divisions in the c2p, the same iterates.
  * Results agree with the plain mode to rounding.  Which cells the aux pass
  * and linop_apply write is chosen separately, by params.ranges
  * (grb_ranges_kind). */
